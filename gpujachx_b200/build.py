@@ -33,7 +33,7 @@ X1 = os.path.join(LIBDIR, "x1")
 PP = os.path.join(LIBDIR, "libgjx_pp.so")
 
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
-NVCC_FLAGS = ARCH + ["-lineinfo", "-O3", "--fmad=false", "-std=c++17", "-Xcompiler", "-fPIC",
+NVCC_FLAGS = ARCH + ["--split-compile=0", "-lineinfo", "-O3", "--fmad=false", "-std=c++17", "-Xcompiler", "-fPIC",
                      "-I" + os.path.join(ROOT, "include"), "-I" + CSRC]
 
 LIB_SOURCES = ["gjx_kernels.cu", "gjx_split.cu", "gjx_host.cpp", "gjx_noalloc.cu", "gjx_h5abi.cpp", "h5mini.cpp"]
@@ -112,16 +112,16 @@ def build_strat(ref_root: str | None = None, force: bool = False, verbose: bool 
     they are consumed unchanged, as the reference's own strat/proc_*-lnx.sh
     does, with the same exported symbol names.  The rowcyc and colcyc tables
     of orders 960 and 1024, which the reference does not ship, are added by
-    its doubling construction (strat_gen).
+    its doubling construction (strat_gen).  Without a reference tree the
+    families are built whole by strat_gen, for the orders it gives.
     """
     ref_root = ref_root or os.environ.get("GJX_REF_ROOT", "")
     sdir = os.path.join(ref_root, "strat") if ref_root else ""
     if not force and os.path.exists(STRAT):
         return STRAT
-    if not sdir or not os.path.isdir(sdir):
-        if os.path.exists(STRAT):
-            return STRAT
-        raise FileNotFoundError(f"no strategy tables (set GJX_REF_ROOT to the reference tree) and no prebuilt {STRAT}")
+    have_ref = bool(sdir) and os.path.isdir(sdir)
+    if not have_ref and os.path.exists(STRAT):
+        return STRAT
     os.makedirs(LIBDIR, exist_ok=True)
     work = tempfile.mkdtemp(prefix="gjx_strat_")
     try:
@@ -148,8 +148,11 @@ def build_strat(ref_root: str | None = None, force: bool = False, verbose: bool 
 
         from . import strat_gen
         with ThreadPoolExecutor(max_workers=len(STRAT_FAMILIES)) as ex:
-            objs = list(ex.map(one, STRAT_FAMILIES))
-            objs += list(ex.map(ext, sorted(strat_gen.extension_sources(sdir).items())))
+            if have_ref:
+                objs = list(ex.map(one, STRAT_FAMILIES))
+                objs += list(ex.map(ext, sorted(strat_gen.extension_sources(sdir).items())))
+            else:
+                objs = list(ex.map(ext, sorted(strat_gen.family_sources().items())))
         tmp = STRAT + ".tmp"
         _run(["gcc", "-shared", "-o", tmp] + objs, verbose)
         os.replace(tmp, STRAT)

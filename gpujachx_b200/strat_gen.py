@@ -1,6 +1,8 @@
-"""Outer strategy tables beyond the reference's largest order (896 blocks,
-N = 14336 columns): the rowcyc and colcyc tables of orders 960 and 1024
-(N = 15360 and 16384), built by the reference's own doubling construction
+"""Strategy tables that a construction gives.
+
+Outer tables beyond the reference's largest order (896 blocks, N = 14336
+columns): the rowcyc and colcyc tables of orders 960 and 1024 (N = 15360 and
+16384), built by the reference's own doubling construction
 (strat/n2n/n2n.sh.cpp:41-129) from its tables of orders 480 and 512.
 
 The construction, for an order-n table T of n-1 parallel steps of n/2
@@ -14,6 +16,18 @@ Every pair of blocks meets once per sweep and each step is a perfect
 matching, as in T.  The reference's tables of every order 2n <= 896 whose
 half it also ships are this doubling of it (all 112 of them;
 tests/test_strat_doubling.py checks it against the tables in strat.so).
+
+Where the reference tree is not at hand, the families are built whole
+(family_sources).  The cyclic ones for the orders 2^k, 3 2^k, 5 2^k and 7 2^k:
+a base of order 2, 6, 10 or 14, doubled; the rowcyc (colcyc) base is the first
+complete set of perfect matchings that a backtracking search finds when it
+takes the pairs in row-cyclic (column-cyclic) order, and cycwor (cycloc) is
+rowcyc (colcyc) with its steps reversed.  BrentL is the ordering of R. P. Brent
+and F. T. Luk (1985), mmstep the modulus ordering with the two indices that
+meet themselves paired (n steps).  The recorded outputs of the reference pin
+these tables: rowcyc, colcyc and cycloc of orders 12 and 32, cycwor of orders 2
+to 512 among them 12, 20, 24 and 28, BrentL and mmstep of orders 16 and 32 give
+its bits (tests/test_oracle_golden.py).
 
 Used by build.build_strat; the generated tables get the reference's symbol
 names (rowcyc00960, ...) and element type (unsigned short above 256).
@@ -58,6 +72,105 @@ def double_table(t: np.ndarray, family: str) -> np.ndarray:
         second[:, 0::2, 0], second[:, 0::2, 1] = 2 * i + 1, 2 * j
         second[:, 1::2, 0], second[:, 1::2, 1] = 2 * i, 2 * j + 1
     return out
+
+
+def base_table(n: int, family: str) -> np.ndarray:
+    """The order-n table (n = 2 odd) that a backtracking search finds first,
+    its steps filled with the pairs in row-cyclic (rowcyc: 01 02 .. 12 ..) or
+    column-cyclic (colcyc: 01 02 12 03 ..) order."""
+    if family == "rowcyc":
+        order = [(i, j) for i in range(n) for j in range(i + 1, n)]
+    else:
+        order = [(i, j) for j in range(n) for i in range(j)]
+    used: set = set()
+    steps: list = []
+
+    def matchings(start, busy, m):
+        if len(m) == n // 2:
+            yield list(m)
+            return
+        for k in range(start, len(order)):
+            i, j = order[k]
+            if order[k] in used or i in busy or j in busy:
+                continue
+            yield from matchings(k + 1, busy | {i, j}, m + [order[k]])
+
+    def search():
+        if len(steps) == n - 1:
+            return True
+        for m in matchings(0, frozenset(), []):
+            steps.append(m)
+            used.update(m)
+            if search():
+                return True
+            steps.pop()
+            used.difference_update(m)
+        return False
+
+    if not search():
+        raise ValueError(f"no table of order {n}")
+    return np.array(steps, dtype=np.int64)
+
+
+def cyclic_table(family: str, n: int) -> np.ndarray:
+    """The order-n table of a cyclic family (rowcyc, colcyc, cycwor, cycloc)."""
+    fwd = {"cycwor": "rowcyc", "cycloc": "colcyc"}.get(family, family)
+    b = n
+    while b % 4 == 0:
+        b //= 2
+    t = base_table(b, fwd)
+    while 2 * t.shape[1] < n:
+        t = double_table(t, fwd)
+    return t if fwd == family else t[::-1]
+
+
+def brent_luk_table(n: int) -> np.ndarray:
+    """n - 1 steps: two rows of n/2 indices, paired by column; from step to
+    step the first index stays and the others move one place around."""
+    top, bottom = list(range(0, n, 2)), list(range(1, n, 2))
+    steps = []
+    for _ in range(n - 1):
+        steps.append([(min(p), max(p)) for p in zip(top, bottom)])
+        top, bottom = [top[0], bottom[0]] + top[1:-1], bottom[1:] + top[-1:]
+    return np.array(steps, dtype=np.int64)
+
+
+def modulus_table(n: int) -> np.ndarray:
+    """n steps, s = n - 1, 0, 1, ..., n - 2: the pairs i + j = s (mod n), and for
+    even s the two i with 2 i = s (mod n) paired with each other."""
+    steps = []
+    for t in range(n):
+        s = (n - 1 + t) % n
+        pairs = [(i, (s - i) % n) for i in range(n) if i < (s - i) % n]
+        if s % 2 == 0:
+            pairs.append((s // 2, s // 2 + n // 2))
+        steps.append(pairs)
+    return np.array(steps, dtype=np.int64)
+
+
+def family_tables():
+    """(family, n, table) of every table that is built without a reference tree."""
+    orders = sorted(b << k for b in (2, 6, 10, 14) for k in range(10) if b << k <= 1024)
+    for fam in ("rowcyc", "colcyc", "cycwor", "cycloc"):
+        for n in orders:
+            if n <= 896 or fam in FAMILIES:
+                yield fam, n, cyclic_table(fam, n)
+    for n in range(16, 897, 16):
+        yield "BrentL", n, brent_luk_table(n)
+        yield "mmstep", n, modulus_table(n)
+
+
+def family_sources() -> dict[str, str]:
+    """{file name: assembler source} of every table of family_tables."""
+    out: dict[str, str] = {}
+    for fam, n, t in family_tables():
+        name, t = "%s%05u" % (fam, n), t.ravel()
+        word = ".byte" if n <= 256 else ".short"
+        data = "\n".join("\t%s %s" % (word, ",".join(map(str, t[i:i + 64]))) for i in range(0, t.size, 64))
+        out[fam + ".s"] = out.get(fam + ".s", "\t.data\n") + (
+            "\t.globl %s\n\t.type %s, @object\n\t.balign 16\n%s:\n%s\n\t.size %s, .-%s\n"
+            % (name, name, name, data, name, name))
+    return {k: v + '\t.section .note.GNU-stack,"",@progbits\n' for k, v in out.items()}
 
 
 def c_source(family: str, n: int, t: np.ndarray) -> str:
