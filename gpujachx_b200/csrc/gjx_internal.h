@@ -113,8 +113,6 @@ cudaError_t make_gram_map(CUtensorMap *tm, const double *base, unsigned nrow, un
 // device error codes written to *err
 enum : int { kErrWaitTimeout = 1 };
 
-size_t l1_smem_bytes();
-size_t batch2_smem_bytes();
 cudaError_t l1_configure();
 cudaError_t launch_l1_step(bool sort, bool accv, const StepParams &p, cudaStream_t s);
 // CTAs per block pair for `pairs` pairs per step on the current device
