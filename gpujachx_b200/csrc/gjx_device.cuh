@@ -46,8 +46,9 @@ __device__ __forceinline__ double pow2(const int k) { return __longlong_as_doubl
 
 // 1/sqrt(a) rounded to nearest.  Our own method.  Scale a = f * 4^k with
 // f in [1, 4), so that 1/sqrt(f) = Y * 2^-53 lies in (1/2, 1) with Y a
-// 53-bit integer after rounding.  From the hardware-assisted estimate y:
-//   * fast path (after P. Markstein, "IA-64 and Elementary Functions"):
+// 53-bit integer after rounding.  From rsqrt()'s value y (here in the whole
+// method; rsqrt_try below is the usual way):
+//   * mostly (after P. Markstein, "IA-64 and Elementary Functions"):
 //     e = 1 - f y^2 by two FMAs on y^2 = yh + yl (error below 2^-103), then
 //     1/sqrt(f) = y (1 + e/2 + O(e^2)); in ulps the correction is
 //     d = 2^53 y e / 2 within 2^-48, so Y = y 2^53 + rint(d) unless d lies
@@ -106,48 +107,115 @@ static __device__ __noinline__ double rsqrt_rn_full(const double a)
   return Yd * pow2(-53 - kk); // exact scaling into the normal range
 }
 
-// Fast path: the estimate from the hardware approximation (relative error
-// about 2^-20, measured) refined by one second-order Newton step to about
-// an ulp, then the same rounding decision as rsqrt_rn_full (after Markstein).
-// The residual e = 1 - f y^2 is formed from a and the unscaled estimate ya
-// (f y^2 = a ya^2: the power-of-4 scalings cancel), so the scaling of y into
-// (1/2, 1] runs beside it; Y = rint(y 2^53 + d) comes from one FMA whose
-// result lies in [2^52, 2^53), where doubles are the integers.  Powers of 4
-// (f = 1) give 2^-kk exactly.  Whatever the decision cannot settle -- signs,
-// zeros, subnormals, inf, NaN, exponents beyond +-960 (where a ya^2 could
-// leave the normal range) and the rare ambiguous roundings -- goes to
-// rsqrt_rn_full in one branch at the end (the fast path's values for those
-// inputs are discarded), so the result is the correctly rounded 1/sqrt(a)
-// either way.
+// ---------------------------------------------------------------------------
+// Correctly rounded reciprocal square root, quotient, reciprocal and square
+// root without branches.  Each takes the hardware's estimate (rsqrt.approx /
+// rcp.approx, relative error about 2^-20, measured), corrects it, and PROVES
+// the result; ok is false when the proof fails -- almost never for the
+// operands of a rotation, always for zeros, infinities, NaN, subnormals and
+// results that are a power of 2 (where the spacing halves below) -- and the
+// caller then takes the IEEE operation.  Without branches the chains of a
+// rotation overlap, which calls of the IEEE operations (each with a branch to
+// its special cases) do not.  The proofs compare high words as integers
+// (hi(|x|) < hi(y) implies |x| < y), so they cost the FP64 pipe, which the
+// warps of a sub-partition share, one or two operations each.
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ int hi_abs(const double a) { return __double2hiint(a) & 0x7FFFFFFF; }
+__device__ __forceinline__ int hi_binade(const double a) { return __double2hiint(a) & 0x7FF00000; }
+__device__ __forceinline__ bool pow2_significand(const double a)
+{
+  return !((__double2hiint(a) & 0xFFFFF) | __double2loint(a));
+}
+
+__device__ __forceinline__ double rsqrt_estimate(const double a)
+{
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(a));
+  return __hiloint2double(__double2hiint(y), 0);
+}
+
+// The estimate y0 has no low word, so y0^2 is exact and the residual e = 1 -
+// a y0^2 takes one FMA; 1/sqrt(a) = y0 (1 - e)^(-1/2) = y0 + (y0 e) (1/2 + 3/8 e
+// + 5/16 e^2 + 35/128 e^3), the next term below 2^-90 (|e| < 2^-18 is checked).
+// The correction is known to 2^-16 of half an ulp of the result c, so c, its
+// sum with y0 rounded once, is 1/sqrt(a) rounded to nearest if it differs from
+// the unrounded sum by less than (1 - 2^-15) / 2 ulp (c - y0 is exact).  The
+// caller sees to a within 2^+-960, where y0^2 and a y0^2 stay normal.
+// A chain of 7 operations: 100 cycles (191 before, with the estimate refined to
+// an ulp first).
+__device__ __forceinline__ double rsqrt_try(const double a, bool &ok)
+{
+  const double y0 = rsqrt_estimate(a);
+  const double e = __fma_rn(-a, y0 * y0, 1.0);
+  const double ye = y0 * e;
+  const double w = __fma_rn(e * e, __fma_rn(0.2734375, e, 0.3125), __fma_rn(0.375, e, 0.5));
+  const double c = __fma_rn(ye, w, y0);
+  const double z = __fma_rn(ye, w, y0 - c);
+  ok = (hi_abs(z) < hi_binade(c) - (53 << 20) - 64) && !pow2_significand(c) && (hi_abs(e) < ((1023 - 18) << 20));
+  return c;
+}
+
+// h / a and 1 / a: the quotient to 2^-40 by one Newton step, then its residual
+// (after P. Markstein, "IA-64 and Elementary Functions").  q is the quotient
+// rounded to nearest if |h - a q| < |a| ulp(q) / 2; the residual is rounded
+// once, which the comparison of high words covers.  The caller sees to
+// |h| >= 2^-900 (or zero).
+__device__ __forceinline__ bool quotient_ok(const double rho, const double a, const double q)
+{
+  return (hi_abs(rho) < hi_abs(a) + (hi_binade(q) - ((1023 + 53) << 20))) && !pow2_significand(q);
+}
+
+__device__ __forceinline__ double rcp_estimate(const double a)
+{
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(a));
+  return y;
+}
+
+__device__ __forceinline__ double div_try(const double h, const double a, bool &ok)
+{
+  const double y0 = rcp_estimate(a), q0 = h * y0;
+  const double e = __fma_rn(-a, y0, 1.0);
+  const double y1 = __fma_rn(y0, e, y0), q1 = __fma_rn(q0, e, q0);
+  const double q = __fma_rn(__fma_rn(-a, q1, h), y1, q1);
+  ok = quotient_ok(__fma_rn(-a, q, h), a, q);
+  return q;
+}
+
+__device__ __forceinline__ double rcp_try(const double a, bool &ok)
+{
+  const double y0 = rcp_estimate(a);
+  const double y1 = __fma_rn(y0, __fma_rn(-a, y0, 1.0), y0);
+  const double t = __fma_rn(__fma_rn(-a, y1, 1.0), y1, y1);
+  ok = quotient_ok(__fma_rn(-a, t, 1.0), a, t);
+  return t;
+}
+
+// sqrt(x): sqrt(x) and 1 / (2 sqrt(x)) to 2^-39 by one step, then the residual;
+// s is sqrt(x) rounded to nearest if |x - s^2| < s ulp(s)
+__device__ __forceinline__ double sqrt_try(const double x, bool &ok)
+{
+  const double y0 = rsqrt_estimate(x);
+  const double g0 = x * y0, h0 = 0.5 * y0;
+  const double r0 = __fma_rn(-g0, h0, 0.5);
+  const double g1 = __fma_rn(g0, r0, g0), h1 = __fma_rn(h0, r0, h0);
+  const double s = __fma_rn(__fma_rn(-g1, g1, x), h1, g1);
+  const double rho = __fma_rn(-s, s, x);
+  ok = (hi_abs(rho) < hi_abs(s) + (hi_binade(s) - ((1023 + 52) << 20))) && !pow2_significand(s);
+  return s;
+}
+
+// rsqrt_rn: the fast path, and rsqrt_rn_full for what it does not settle
+__device__ __forceinline__ bool rsqrt_range(const double a) // 2^-960 <= a < 2^960
+{
+  return (unsigned)(__double2hiint(a) - (63 << 20)) < (1920u << 20);
+}
+
 __device__ __forceinline__ double rsqrt_rn(const double a)
 {
-  const unsigned long long bits = (unsigned long long)__double_as_longlong(a);
-  const unsigned long long ef = bits >> 52; // sign and exponent field
-  double y0;
-  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y0) : "d"(a));
-  const double h0 = a * y0;
-  const double r0 = __fma_rn(-h0, y0, 1.0);
-  const double ya = __fma_rn(y0 * r0, __fma_rn(0.375, r0, 0.5), y0); // y0 (1 + r0/2 + 3 r0^2/8)
-  const int eu = (int)ef - 1023;
-  const int kk = (eu & ~1) / 2; // a = f * 4^kk, f in [1, 4)
-  // e = 1 - f y^2 with y^2 = yh + yl split exactly (y = ya 2^kk, f = a 4^-kk)
-  const double yh = ya * ya;
-  const double yl = __fma_rn(ya, ya, -yh);
-  const double e = __fma_rn(-a, yl, __fma_rn(-a, yh, 1.0));
-  const double y52 = ya * pow2(52 + kk); // y 2^52 (exact), beside the residual
-  // the correction in ulps of y, (y (e/2)) 2^53 = (y 2^52) e
-  const double d = y52 * e;
-  // Y = y 2^53 + rint(d): y 2^53 is an integer, and the FMA rounds the sum
-  // in [2^52, 2^53) to an integer (ties cannot occur: they are refused below)
-  const double Yd = __fma_rn(y52, 2.0, d);
-  const double dr = Yd - 2.0 * y52; // rint(d), exact
-  // a power of 4 (f = 1, e.g. 1 + t^2 = 1 for a tiny rotation angle): 2^-kk exactly
-  const bool p4 = !(bits & 0xFFFFFFFFFFFFFull) && !(eu & 1);
-  const double res = p4 ? pow2(-kk) : Yd * pow2(-53 - kk);
-  if ((ef - 1ull > 2045ull) || (eu < -960) || (eu > 960) ||
-      (!p4 && (!(fabs(d) < 0x1.0p50) || fabs(d - dr) > 0.5 - 0x1.0p-40 || Yd >= pow2(53) || Yd < pow2(52))))
-    return rsqrt_rn_full(a);
-  return res;
+  bool ok;
+  const double c = rsqrt_try(a, ok);
+  return (ok && rsqrt_range(a)) ? c : rsqrt_rn_full(a);
 }
 
 // ---------------------------------------------------------------------------
@@ -165,41 +233,11 @@ __device__ __forceinline__ double sum32(double v)
 }
 
 // ---------------------------------------------------------------------------
-// 2x2 rotations (share/device_code_common_rotate.hpp:16-64, USE_RSQRT form).
-// Return 1 for a "big" rotation (c != 1), 0 otherwise.
+// 2x2 rotations (share/device_code_common_rotate.hpp:16-64, USE_RSQRT form):
+// the three cases of each kind are selects of values that every lane
+// computes, so the lanes that evaluate different rotations never diverge.
+// "big" rotations (c != 1) are counted.
 // ---------------------------------------------------------------------------
-// The three cases of each are evaluated without branching (the operands of
-// the case that applies are selected, then the same operations run), so the
-// 16 lanes that compute 16 rotations at once never diverge.
-__device__ __forceinline__ int rotT(const double Apq, const double Dp, const double Dq, double &c, double &t)
-{
-  const double h = Dq - Dp;
-  const double ct2 = __ddiv_rn(h, Apq * 2.0);
-  const double CT2 = fabs(ct2);
-  const bool small = CT2 < kSqrtHeps, large = CT2 >= kSqrt2Heps;
-  const double cot_mid = CT2 + __dsqrt_rn(__fma_rn(CT2, CT2, 1.0));
-  const double cot = small ? (CT2 + 1.0) : (large ? (CT2 * 2.0) : cot_mid);
-  t = copysign(__drcp_rn(cot), ct2);
-  const double cr = rsqrt_rn(__fma_rn(t, t, 1.0));
-  c = large ? 1.0 : cr;
-  return small ? 1 : (large ? 0 : (cr < 1.0));
-}
-
-__device__ __forceinline__ int rotH(const double Apq, const double Dp, const double Dq, double &c, double &t)
-{
-  const double h = Dq + Dp;
-  const double ct2 = -__ddiv_rn(h, Apq * 2.0);
-  const double CT2 = fabs(ct2);
-  const bool large = CT2 >= kSqrt2Heps, mid = !large && (CT2 > 1.0);
-  const double cot_mid = CT2 + __dsqrt_rn(__fma_rn(CT2, CT2, -1.0));
-  const double cot = large ? (CT2 * 2.0) : cot_mid;
-  const double tt = copysign(__drcp_rn(cot), ct2);
-  const double cr = rsqrt_rn(__fma_rn(-tt, tt, 1.0));
-  c = large ? 1.0 : (mid ? cr : kCoshIFix);
-  t = (large || mid) ? tt : kTanh1Fix;
-  return large ? 0 : (mid ? (cr > 1.0) : 1);
-}
-
 // one inner rotation, as the lanes that compute it hand it to those that apply it
 struct Rot {
   double c, t, t_;
@@ -207,13 +245,13 @@ struct Rot {
   int scale, swap;
 };
 
-// rotT for the lanes with trig, rotH for the others, in one chain.  The two
-// formulas take the same operations up to signs -- Dq - Dp is Dq + (-Dp)
-// exactly, the quotient negated, +1 or -1 under the square root, t t + 1 or
-// -t t + 1 under the reciprocal square root -- and their special cases are
-// selects, so each lane gets exactly the operations of its own formula while
-// a warp whose lanes need both kinds runs one chain of divides and square
-// roots instead of two.
+// rotT for the lanes with trig, rotH for the others, in one chain, by the
+// IEEE operations.  The two formulas take the same operations up to signs --
+// Dq - Dp is Dq + (-Dp) exactly, the quotient negated, +1 or -1 under the
+// square root, t t + 1 or -t t + 1 under the reciprocal square root -- and
+// their special cases are selects, so each lane gets exactly the operations
+// of its own formula while a warp whose lanes need both kinds runs one chain
+// of divides and square roots instead of two.
 __device__ __forceinline__ int rotTH(const bool trig, const double Apq, const double Dp, const double Dq, double &c,
                                      double &t)
 {
@@ -233,17 +271,68 @@ __device__ __forceinline__ int rotTH(const bool trig, const double Apq, const do
   return trig ? (small ? 1 : (large ? 0 : (cr < 1.0))) : (large ? 0 : (mid ? (cr > 1.0) : 1));
 }
 
-// rotT (trig) or rotH; when the lanes of the warp need different kinds, the
-// merged chain of rotTH (each is a long dependent chain of divisions and
-// square roots)
-__device__ __forceinline__ int rot_either(const bool trig, const double Apq, const double Dp, const double Dq,
-                                          double &c, double &t)
+// the relative test and the rotation by the IEEE operations: the lanes whose
+// fast path could not prove a value (c | t | ts | b)
+struct RotRaw {
+  double c, t;
+  int ts, b;
+};
+static __device__ __noinline__ RotRaw rot_ieee(const bool trig, const double Apq, const double Dp, const double Dq)
 {
-  if (__all_sync(0xffffffffu, trig))
-    return rotT(Apq, Dp, Dq, c, t);
-  if (__all_sync(0xffffffffu, !trig))
-    return rotH(Apq, Dp, Dq, c, t);
-  return rotTH(trig, Apq, Dp, Dq, c, t);
+  RotRaw r;
+  r.ts = !(fabs(Apq) < ((__dsqrt_rn(Dp) * __dsqrt_rn(Dq)) * kMyTol));
+  r.b = rotTH(trig, Apq, Dp, Dq, r.c, r.t);
+  return r;
+}
+
+// The same values by the branch-free operations above, in one block of
+// independent chains.  MIXED: some lanes of the warp are hyperbolic.
+// The relative test |Apq| < RN(RN(sqrt Dp) RN(sqrt Dq)) tol is decided by Apq^2
+// against Dp Dq tol^2 (tol^2 = 2^-101 to 2^-52), without the two square roots:
+// the high words order as the rounded sides do when they differ by 2 or more
+// (2^-20 relatively, the roundings 2^-49).
+// The reciprocal root of f = 1 +- t^2 for g = 1 - f (exact), |g| < 2^-30, is
+// 1 + g (1/2 + 3/8 g) rounded once.  There 1 + g/2 is a representable number, a
+// midpoint or a quarter of the spacing, and the true value lies above it by
+// 3/8 g^2 + ...: the computed sum lies above it too (1/2 is taken one ulp larger,
+// for the g whose 3/8 g is lost) and by less than a quarter of the spacing, so
+// it rounds as the true value does; for g < 0 1 + g/2 is representable and
+// both round to it.
+// Measured (inner_rot, one warp; two warps per sub-partition): 451 and 538
+// cycles, against 715 and 775 with the IEEE operations one after the other.
+// bad: a value that this lane's rotation uses is not proved, or the test is
+// too close to call, or Dp Dq is outside 2^+-800 (within it no intermediate
+// result above leaves the normal range unnoticed).
+template <bool MIXED>
+__device__ __forceinline__ RotRaw rot_try(const bool trig, const double Apq, const double Dp, const double Dq,
+                                          bool &bad)
+{
+  RotRaw r;
+  const int hP = __double2hiint(Dp * Dq), dh = __double2hiint(Apq * Apq) - (hP - (101 << 20));
+  const bool sure = ((unsigned)(hP - (223 << 20)) < (1600u << 20)) && ((unsigned)(dh + 1) > 2u);
+  r.ts = dh > 0;
+
+  const double h = Dq + ((!MIXED || trig) ? -Dp : Dp);
+  bool ok_q, ok_s, ok_t, ok_c;
+  const double qt = div_try(h, Apq * 2.0, ok_q);
+  const double ct2 = (!MIXED || trig) ? qt : -qt;
+  const double CT2 = fabs(ct2);
+  const unsigned long long cbits = (unsigned long long)__double_as_longlong(CT2);
+  const bool large = cbits >= (unsigned long long)__double_as_longlong(kSqrt2Heps);
+  const bool small = (!MIXED || trig) && (cbits < (unsigned long long)__double_as_longlong(kSqrtHeps));
+  const bool fixed = MIXED && !trig && (cbits <= 0x3FF0000000000000ull); // rotH's last case: constants
+  const double alt = small ? 1.0 : CT2; // cot = CT2 + 1, 2 CT2 or CT2 + sqrt(CT2^2 +- 1)
+  const double sq = sqrt_try(__fma_rn(CT2, CT2, (!MIXED || trig) ? 1.0 : -1.0), ok_s);
+  const double t = rcp_try(CT2 + ((small || large) ? alt : sq), ok_t);
+  const double f = __fma_rn((!MIXED || trig) ? t : -t, t, 1.0), g = 1.0 - f;
+  const double cr = rsqrt_try(f, ok_c);
+  const bool near1 = hi_abs(g) < ((1023 - 30) << 20);
+  const double c1 = near1 ? __fma_rn(g, __fma_rn(0.375, g, 0x1.0000000000001p-1), 1.0) : cr;
+  r.c = large ? 1.0 : (fixed ? kCoshIFix : c1);
+  r.t = fixed ? kTanh1Fix : copysign(t, ct2);
+  r.b = (unsigned long long)__double_as_longlong(r.c) != 0x3FF0000000000000ull; // c != 1
+  bad = !sure || (r.ts && (!ok_q || (!fixed && (!ok_t || !(large || ((near1 || ok_c) && (small || ok_s)))))));
+  return r;
 }
 
 template <bool SORT>
@@ -251,40 +340,32 @@ __device__ __forceinline__ Rot inner_rot(const double Dp, const double Dq, const
                                          const unsigned q, const int definite, const unsigned npos, unsigned &ts_out,
                                          unsigned &tb_out)
 {
-  // branch-free: the two half-warps handle different pairs, so every choice
-  // below is a select of values computed by both (no divergent paths)
+  // branch-free: the parts of a warp handle different pairs, so every choice
+  // below is a select of values computed by both (no divergent paths); the
+  // rotation is computed whether or not it is applied
+  const int def = definite ? definite : ((p < npos) && (q < npos)) ? +1 : ((p >= npos) && (q >= npos)) ? -1 : 0;
+  bool bad;
+  RotRaw w = (definite || __all_sync(0xffffffffu, def != 0)) ? rot_try<false>(true, Apq, Dp, Dq, bad)
+                                                             : rot_try<true>(def != 0, Apq, Dp, Dq, bad);
+  if (bad)
+    w = rot_ieee(def != 0, Apq, Dp, Dq);
   Rot r;
-  const double Dp_ = __dsqrt_rn(Dp), Dq_ = __dsqrt_rn(Dq), Apq_ = fabs(Apq), Dpq_ = Dp_ * Dq_;
-  const int ts = !(Apq_ < (Dpq_ * kMyTol));
-  int tb;
+  const int ts = w.ts;
+  const double t_ = def ? -w.t : w.t;
+  r.c = ts ? w.c : 1.0;
+  r.t = ts ? w.t : 0.0;
+  r.t_ = ts ? t_ : 0.0;
+  const int tb = ts ? w.b : 0;
+  r.scale = tb;
   if (!SORT) {
-    // the rotation is computed whether or not it is applied (no side
-    // effects), so that its latency overlaps the relative test
-    const bool trig = definite || ((p < npos) && (q < npos)) || ((p >= npos) && (q >= npos));
-    double c, t;
-    const int b = rot_either(trig, Apq, Dp, Dq, c, t);
-    r.c = ts ? c : 1.0;
-    r.t = ts ? t : 0.0;
-    r.t_ = ts ? (trig ? -t : t) : 0.0;
-    tb = ts ? b : 0;
     r.mode = ts;
-    r.scale = tb;
     r.swap = 0;
   }
   else {
-    const int def = definite ? definite : ((p < npos) && (q < npos)) ? +1 : ((p >= npos) && (q >= npos)) ? -1 : 0;
-    double c, t;
-    const int b = rot_either(def != 0, Apq, Dp, Dq, c, t);
-    const double t_ = def ? -t : t;
-    const double Dp2 = __fma_rn(t, Apq, Dp), Dq2 = __fma_rn(t_, Apq, Dq); // used when ts and def
+    const double Dp2 = __fma_rn(w.t, Apq, Dp), Dq2 = __fma_rn(t_, Apq, Dq); // used when ts and def
     const int swp = !((!def) || ((def > 0) && (Dp2 >= Dq2)) || ((def < 0) && (Dp2 <= Dq2)));
     const int order = ((def > 0) && (Dp < Dq)) || ((def < 0) && (Dq < Dp));
-    r.c = ts ? c : 1.0;
-    r.t = ts ? t : 0.0;
-    r.t_ = ts ? t_ : 0.0;
-    tb = ts ? b : 0;
     r.mode = ts ? 1 : (order ? 2 : 0);
-    r.scale = tb;
     r.swap = ts ? swp : 0;
   }
   ts_out = (unsigned)ts;
