@@ -19,8 +19,7 @@
 //      slide through a row window, and all operands come as 16-byte row
 //      pairs.  The shares are exchanged through distributed shared memory,
 //      then one cluster barrier.
-//   2. 32x32 Cholesky by the CTA with a one-column look-ahead: warp 0 updates
-//      and pivots the next column while warps 1-7 update the rest
+//   2. 32x32 Cholesky by one warp, the trailing matrix in registers
 //      (share/device_code_common_Cholesky.hpp:58-158).
 //   3. Inner Jacobi sweep(s) on R: per inner step each warp sums the dot
 //      products of its two pairs by register butterflies in the reference's
@@ -333,68 +332,71 @@ __device__ __forceinline__ bool gram_lane_of(const unsigned rank, const unsigned
 }
 
 // ---------------------------------------------------------------------------
-// Right-looking Cholesky of the lower triangle held in R, by the whole CTA,
-// with a one-column look-ahead: in round k warp 0 updates column k+1 by
-// column k and pivots it (x > k+1: times rsqrt_rn(A(k+1,k+1)), the diagonal
-// its square root) while warps 1..7 update columns k+2..31 by column k,
-// A(x,j) = fma(-A(x,k), A(j,k), A(x,j)) for x >= j.  Every entry receives
-// the reference's operations in the reference's order
-// (share/device_code_common_Cholesky.hpp:58-158); one barrier per column.
+// Right-looking Cholesky of the lower triangle held in R, by one warp with
+// the trailing matrix in registers: lane x holds row x, a[j] = A(x, k + j) in
+// round k.  A round scales column k (x > k: times rsqrt_rn(A(k,k))), then
+// every trailing entry takes A(x,j) = fma(-A(x,k), A(j,k), A(x,j)) and moves
+// one register down, so that a round's indices are constants.  Every entry
+// receives the reference's operations in the reference's order
+// (share/device_code_common_Cholesky.hpp:58-158); entries above the diagonal
+// are computed too and never used.
+// The round's serial chain is the pivot: lane k + 1 updates its own diagonal
+// entry (its factor is its own), one shuffle hands it to all lanes, and its
+// rsqrt_rn runs beside the trailing updates, whose factors A(j,k) come back
+// from shared memory (column k of R, where they belong anyway) by broadcast
+// loads.  The square roots of the diagonal are taken together at the end.
+// No barrier inside.  With a column look-ahead over 8 warps and a barrier per
+// column the pivot's chain was barrier, loads, update, shuffle, reciprocal root
+// and root; this form takes 2 to 5 us less of a step (256x256: 44.8 -> 42.4 us
+// per step, 4096x2048: 132 -> 129.6).
 // Afterwards R = L^T with zeros below the diagonal.
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ void chol_pivot(double *const R, const unsigned j, const unsigned x, const double a)
+// rounds 32 - LIVE .. 32 - LIVE + 7, LIVE columns alive in the first of them
+template <unsigned LIVE>
+__device__ __forceinline__ void chol_rounds(double *const R, const unsigned x, double (&a)[32], double &rs,
+                                            double &diag)
 {
-  const double ajj = __shfl_sync(0xffffffffu, a, j);
-  const double rs = rsqrt_rn(ajj), sq = __dsqrt_rn(ajj);
-  if (x > j)
-    E32(R, x, j) = a * rs;
-  else if (x == j)
-    E32(R, j, j) = sq;
+#pragma unroll 1
+  for (unsigned k = 32u - LIVE; k < 40u - LIVE; ++k) {
+    const double l = a[0] * rs;
+    if (x == k)
+      diag = a[0];
+    double *const col = R + k * 32u;
+    if (x > k)
+      col[x] = l;
+    // the next pivot (for k = 31 the values below are past the last column and unused)
+    const double pv = __shfl_sync(0xffffffffu, __fma_rn(-l, l, a[1]), (k + 1u) & 31u);
+    bool ok;
+    rs = rsqrt_try(pv, ok);
+    __syncwarp();
+#pragma unroll
+    for (unsigned j = 1u; j < LIVE; ++j)
+      a[j - 1u] = __fma_rn(-l, col[k + j], a[j]);
+    if (!(ok && rsqrt_range(pv)) && k + 1u < 32u)
+      rs = rsqrt_rn_full(pv);
+  }
 }
 
 // by a group of NW warps (thread gt of the group, named barrier bar): the
-// group's warp 0 pivots, warps 1..NW-1 update the trailing columns
+// group's warp 0 factors, all transpose
 template <unsigned NW>
 __device__ __forceinline__ void chol32_grp(double *const R, const unsigned gt, const unsigned bar)
 {
-  const unsigned w = gt >> 5, x = gt & 31u;
-  if (w == 0u)
-    chol_pivot(R, 0u, x, E32(R, x, 0u));
-  bar_sync(bar, NW * 32u);
-#pragma unroll 1
-  for (unsigned k = 0u; k + 1u < 32u; ++k) {
-    if (w == 0u) {
-      const unsigned j = k + 1u;
-      double a = E32(R, x, j);
-      if (x >= j)
-        a = __fma_rn(-E32(R, x, k), E32(R, j, k), a);
-      chol_pivot(R, j, x, a);
-    }
-    else {
-      // the columns of a round are independent: four at a time, so that
-      // their shared-memory loads overlap (each entry's operations unchanged)
-      const double xk = -E32(R, x, k);
-      unsigned j = k + 1u + w;
-#pragma unroll 1
-      for (; j + 3u * (NW - 1u) < 32u; j += 4u * (NW - 1u)) {
-        double ajk[4], axj[4];
+  if (gt < 32u) {
+    const unsigned x = gt;
+    double a[32], diag = 0.0;
 #pragma unroll
-        for (unsigned u = 0u; u < 4u; ++u) {
-          ajk[u] = E32(R, j + u * (NW - 1u), k);
-          axj[u] = E32(R, x, j + u * (NW - 1u));
-        }
-#pragma unroll
-        for (unsigned u = 0u; u < 4u; ++u)
-          if (x >= j + u * (NW - 1u))
-            E32(R, x, j + u * (NW - 1u)) = __fma_rn(xk, ajk[u], axj[u]);
-      }
-#pragma unroll 1
-      for (; j < 32u; j += NW - 1u)
-        if (x >= j)
-          E32(R, x, j) = __fma_rn(xk, E32(R, j, k), E32(R, x, j));
-    }
-    bar_sync(bar, NW * 32u);
+    for (unsigned j = 0u; j < 32u; ++j)
+      a[j] = E32(R, x, j);
+    double rs = rsqrt_rn(__shfl_sync(0xffffffffu, a[0], 0));
+    __syncwarp();
+    chol_rounds<32u>(R, x, a, rs, diag);
+    chol_rounds<24u>(R, x, a, rs, diag);
+    chol_rounds<16u>(R, x, a, rs, diag);
+    chol_rounds<8u>(R, x, a, rs, diag);
+    E32(R, x, x) = __dsqrt_rn(diag);
   }
+  bar_sync(bar, NW * 32u);
   constexpr unsigned NV = 1024u / (NW * 32u);
   double v[NV];
 #pragma unroll
