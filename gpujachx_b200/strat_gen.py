@@ -18,8 +18,8 @@ half it also ships are this doubling of it (all 112 of them;
 tests/test_strat_doubling.py checks it against the tables in strat.so).
 
 Where the reference tree is not at hand, the families are built whole
-(family_sources).  The cyclic ones for the orders 2^k, 3 2^k, 5 2^k and 7 2^k:
-a base of order 2, 6, 10 or 14, doubled; the rowcyc (colcyc) base is the first
+(family_sources).  The cyclic ones for the orders 2^k, 3 2^k, 5 2^k, 7 2^k and
+9 2^k: a base of order 2, 6, 10, 14 or 18, doubled; the rowcyc (colcyc) base is the first
 complete set of perfect matchings that a backtracking search finds when it
 takes the pairs in row-cyclic (column-cyclic) order, and cycwor (cycloc) is
 rowcyc (colcyc) with its steps reversed.  BrentL is the ordering of R. P. Brent
@@ -150,7 +150,7 @@ def modulus_table(n: int) -> np.ndarray:
 
 def family_tables():
     """(family, n, table) of every table that is built without a reference tree."""
-    orders = sorted(b << k for b in (2, 6, 10, 14) for k in range(10) if b << k <= 1024)
+    orders = sorted(b << k for b in (2, 6, 10, 14, 18) for k in range(10) if b << k <= 1024)
     for fam in ("rowcyc", "colcyc", "cycwor", "cycloc"):
         for n in orders:
             if n <= 896 or fam in FAMILIES:
