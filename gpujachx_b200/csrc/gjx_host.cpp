@@ -229,7 +229,7 @@ int run_sweeps_core(const unsigned routine, const unsigned nrow, const unsigned 
   p.s0steps = g_strat.steps0;
   p.nswp0 = blk_ori ? 1u : gjx::kNSweep;
   p.gdefinite = (nplus ? ((nplus < ncol) ? 0 : +1) : -1);
-  p.split = gjx::l1_split(p.pairs);
+  p.split = gjx::l1_split(p.pairs, nrow);
   int mode = g_sweep_mode;
   const auto tuned = g_tuned.find(TuneKey{routine, nrow, ncol, nplus});
   if (tuned != g_tuned.end()) {
@@ -1286,7 +1286,7 @@ void gjx_set_sweep_mode(const int mode)
 void gjx_set_split(const unsigned n)
 {
   std::lock_guard<std::mutex> lk(g_mtx);
-  g_split = (n == 1u || n == 2u || n == 4u) ? n : 0u;
+  g_split = (n == 1u || n == 2u || n == 4u || n == 8u) ? n : 0u;
 }
 
 void gjx_set_variant(const unsigned v)
@@ -1454,12 +1454,14 @@ int gjx_autotune(const unsigned routine, const unsigned nrow, const unsigned nco
   g_verbose = 0;
   g_sweep_cap = sweeps ? sweeps : 1u;
   float best = 3.0e38f;
-  std::pair<unsigned, int> pick{gjx::l1_split(g_strat.pairs1), 0};
+  std::pair<unsigned, int> pick{gjx::l1_split(g_strat.pairs1, nrow), 0};
   int rc = 0;
-  for (unsigned split : {1u, 2u, 4u}) {
-    if (split * g_strat.pairs1 > 148u * 8u)
+  for (unsigned split : {1u, 2u, 4u, 8u}) {
+    if (split * g_strat.pairs1 > ((split == 8u) ? 148u : 148u * 8u))
       continue;
     for (int mode : {0, 1}) {
+      if (mode == 1 && split == 8u) // per step only
+        continue;
       g_split = split;
       g_sweep_mode = mode;
       unsigned swp;

@@ -30,7 +30,7 @@ struct alignas(64) StepParams {
   unsigned s0steps;             // inner steps (31, or 32 for mmstep)
   unsigned nswp0;               // inner sweeps per block pair (1 or 30)
   int gdefinite;                // +1 J = I, -1 J = -I, 0 mixed signs
-  unsigned split;               // CTAs per block pair (a cluster): 1, 2 or 4
+  unsigned split;               // CTAs per block pair (a cluster): 1, 2, 4 or 8
   unsigned width;               // with split 1: block pairs per CTA, 1 or 2 (l1_step2_kernel)
   unsigned steps1;              // outer steps per sweep (persistent sweep kernel)
   unsigned *ver;                // per block: CTAs that have finished writing it this sweep
@@ -115,8 +115,9 @@ enum : int { kErrWaitTimeout = 1 };
 
 cudaError_t l1_configure();
 cudaError_t launch_l1_step(bool sort, bool accv, const StepParams &p, cudaStream_t s);
-// CTAs per block pair for `pairs` pairs per step on the current device
-unsigned l1_split(unsigned pairs);
+// CTAs per block pair for `pairs` pairs per step of an nrow-row matrix on the
+// current device (after l1_configure)
+unsigned l1_split(unsigned pairs, unsigned nrow);
 cudaError_t launch_initD(double *G, double *D, unsigned nrow, unsigned ncol, unsigned nplus, unsigned ldG,
                          cudaStream_t s);
 cudaError_t launch_initV(double *V, unsigned ncol, unsigned ldV, cudaStream_t s);

@@ -266,7 +266,9 @@ cudaError_t l1_configure()
       (e = set_smem<true, true, 1u>(b)) || (e = set_smem<false, false, 2u>(b3)) || (e = set_smem<false, true, 2u>(b3)) ||
       (e = set_smem<true, false, 2u>(b3)) || (e = set_smem<true, true, 2u>(b3)) ||
       (e = set_smem<false, false, 4u>(b3)) || (e = set_smem<false, true, 4u>(b3)) ||
-      (e = set_smem<true, false, 4u>(b3)) || (e = set_smem<true, true, 4u>(b3)))
+      (e = set_smem<true, false, 4u>(b3)) || (e = set_smem<true, true, 4u>(b3)) ||
+      (e = set_smem<false, false, 8u>(b3)) || (e = set_smem<false, true, 8u>(b3)) ||
+      (e = set_smem<true, false, 8u>(b3)) || (e = set_smem<true, true, 8u>(b3)))
     return e;
   return cudaSuccess;
 }
@@ -332,6 +334,8 @@ template <bool S, bool A, unsigned N> static cudaError_t sweep_launch(const Step
 
 bool sweep_kernel_fits(const bool sort, const bool accv, const StepParams &p)
 {
+  if (p.split > 4u) // clusters of 8: one launch per step only
+    return false;
   if (p.split == 4u) {
     if (sort)
       return accv ? sweep_fits<true, true, 4u>(p) : sweep_fits<true, false, 4u>(p);
@@ -364,12 +368,53 @@ cudaError_t launch_l1_sweep(const bool sort, const bool accv, const StepParams &
   return accv ? sweep_launch<false, true, 1u>(p, s) : sweep_launch<false, false, 1u>(p, s);
 }
 
-unsigned l1_split(const unsigned pairs)
+// The largest clusters that are all resident at once, 8 CTAs only from this many
+// rows: below, their thinner Gram shares and fewer update stages do not pay for
+// the wider exchange.  us per call of n = 256, ALG 11, with 8 / 4 CTAs per pair:
+// 256 rows 5256 / 5247, 512: 5470 / 5483, 1024: 5935 / 6444, 4096: 9394 / 10813,
+// 16384: 22471 / 28281.  More clusters than fit at once run in two waves: 34
+// pairs per step (2048 x 1088) take 104 ms with 4 CTAs per pair, 67 ms with 2.
+constexpr unsigned kSplit8Rows = 1024u;
+
+// how many clusters of N CTAs of the step kernel the current device holds at
+// once (a GPC's SMs divide into whole clusters only, so fewer than SMs / N)
+template <unsigned N> static unsigned resident_clusters()
 {
-  int dev = 0, sms = 148;
-  if (cudaGetDevice(&dev) == cudaSuccess)
-    (void)cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  return (4u * pairs <= (unsigned)sms) ? 4u : (2u * pairs <= (unsigned)sms) ? 2u : 1u;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(N);
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = step_smem_bytes(N);
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = N;
+  at[0].val.clusterDim.y = 1;
+  at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  int n = 0;
+  if (cudaOccupancyMaxActiveClusters(&n, l1_step_kernel<true, true, N>, &cfg) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return 0u;
+  }
+  return (unsigned)n;
+}
+
+unsigned l1_split(const unsigned pairs, const unsigned nrow)
+{
+  struct Fit {
+    bool known = false;
+    unsigned c8 = 0u, c4 = 0u, c2 = 0u;
+  };
+  static Fit fits[64]; // by device; the caller holds the library's lock
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev >= 64)
+    return 1u;
+  Fit &f = fits[dev];
+  if (!f.known)
+    f = Fit{true, resident_clusters<8u>(), resident_clusters<4u>(), resident_clusters<2u>()};
+  if (pairs <= f.c8 && nrow >= kSplit8Rows)
+    return 8u;
+  return (pairs <= f.c4) ? 4u : (pairs <= f.c2) ? 2u : 1u;
 }
 
 template <bool S, bool A> static cudaError_t launch2(const StepParams &p, cudaStream_t s)
@@ -401,6 +446,11 @@ cudaError_t launch_l1_step(const bool sort, const bool accv, const StepParams &p
     if (sort)
       return accv ? launch2<true, true>(p, s) : launch2<true, false>(p, s);
     return accv ? launch2<false, true>(p, s) : launch2<false, false>(p, s);
+  }
+  if (n == 8u) {
+    if (sort)
+      return accv ? launch<true, true, 8u>(p, s) : launch<true, false, 8u>(p, s);
+    return accv ? launch<false, true, 8u>(p, s) : launch<false, false, 8u>(p, s);
   }
   if (n == 4u) {
     if (sort)

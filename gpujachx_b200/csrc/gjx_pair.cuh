@@ -3,7 +3,7 @@
 // gjx_batch.cu and gjx_flow.cu).
 //
 // One block pair (i, j) of an outer step is processed by a cluster of NSPLIT
-// CTAs (NSPLIT = 4 or 2 when the step has few pairs, so that more SMs work on
+// CTAs (NSPLIT = 8, 4 or 2 when the step has few pairs, so that more SMs work on
 // each pair; 1 when the pairs already fill the GPU), 256 threads each:
 //
 //   1. Gram matrix of the M x 32 column pair [G_i G_j], lower triangle only
@@ -12,12 +12,9 @@
 //      bank-skewed, zero-padded layout, mbarrier completion, 4 stages of 2
 //      tiles) and computes its share of the 528 entries; every
 //      entry is one FMA chain in the reference's row order
-//      (share/device_code_common_Cholesky.hpp:4-56).  A lane holds the
-//      chains (x0..x0+3, y) of one column y (2-CTA clusters), also of a
-//      second column (one CTA per pair), or (x0, x0+1; y) (4-CTA clusters):
-//      the operands of the x columns are shared by the warp, the y columns
-//      slide through a row window, and all operands come as 16-byte row
-//      pairs.  The shares are exchanged through distributed shared memory,
+//      (share/device_code_common_Cholesky.hpp:4-56).  A lane holds 1 (8-CTA
+//      clusters) to 8 chains (one CTA per pair) of neighbouring columns x and
+//      one or two columns y.  The shares are exchanged through distributed shared memory,
 //      then one cluster barrier.
 //   2. 32x32 Cholesky by one warp, the trailing matrix in registers
 //      (share/device_code_common_Cholesky.hpp:58-158).
@@ -113,223 +110,168 @@ inline size_t step_smem_bytes(const unsigned nsplit)
 #define E32(A, r, c) (A)[(c) * 32u + (r)]
 
 // ---------------------------------------------------------------------------
-// Gram: one 64-row tile (at offset base of the stage) for the 4 entries
-// (x0+u, y), u < 4, of one lane.  Entry (x, y) adds G[r,y]*G[r,x] for
-// r = x, x+1, ..., x+63 (mod 64), the reference's order.  With k = r - x0
-// (0..66, taken mod 64) chain u takes the k in [u, u+63] in increasing order.
-// Operands come in 16-byte pairs of rows (k, k+1), k even (a pair never
-// straddles a piece): one pair of column y and one of each column x0+u per
-// two rows; the pairs of k + 4 are in flight while those of k are used.
+// Gram: one 64-row tile for the XU YU chains (x, y) of a lane, x = X0 + lx XU + u
+// (u < XU), y = y0 + v dy (v < YU).  Chain (x, y) adds G[r,y]*G[r,x] for r = x,
+// x+1, ..., x+63 (mod 64), the reference's order.  With k = r - X0 the chain
+// takes the k in [d, d+63], d = lx XU + u, in increasing order (rows mod 64); lx
+// is below LX (1 or 2), so a block's lanes read the same rows in the same
+// iteration and differ only in the first and last LX XU of them.
+// Operands come in 16-byte pairs of rows (k, k+1), k even, the pairs of k + 4
+// in flight while those of k are used.
+// What bounds it (measured on resident operands): a sub-partition takes in one
+// 16-byte load of a warp in 7 to 8 cycles whatever its addresses, the SM one
+// distinct 128 bytes per half-warp in a cycle, and a chain one FMA in 9.7.  So
+// in the clusters a lane holds few chains of many operands shared, and lanes
+// 2j, 2j+1 share their columns y, all even (odd) lanes their columns x: 8
+// columns y per half-warp, in 8 bank groups.  Cycles per tile of the 3 warps of
+// a CTA: 1x1 643 (8 CTAs), 1x2 735 (4 CTAs), 2x2 1028 (2 CTAs); before, with 32
+// columns y per warp, 2x1 864 (4 CTAs) and 4x1 1306 (2 CTAs).  With one CTA per
+// pair the chains fill 3 warps best as 4x2 with LX = 1 (1897; 2x2 on 4 warps
+// with the diagonal blocks beside other chains measured 25 % slower).
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ void gram_tile(const double *const st, const unsigned base, const unsigned x0,
-                                          const unsigned y, double (&acc)[4])
+template <unsigned XU, unsigned YU, unsigned LX>
+__device__ __forceinline__ void gram_tile(const double *const st, const unsigned X0, const unsigned lx,
+                                          const unsigned y0, const unsigned dy, double (&acc)[XU][YU])
 {
-  const double *const yp = st + base + y * kGramColLd;
-  const double *const xp = st + base + x0 * kGramColLd;
-  double2 Yb[3], Xb[3][4];
+  constexpr unsigned NP = (64u + LX * XU) / 2u; // row pairs: k = 0 .. 63 + LX XU - 1
+  const double *const yp = st + y0 * kGramColLd;
+  const double *const xp = st + (X0 + lx * XU) * kGramColLd;
+  double2 Yb[3][YU], Xb[3][XU];
+  const auto load = [&](const unsigned kp) {
+    const unsigned q = kp % 3u, o = (X0 + 2u * kp) & 63u;
 #pragma unroll
-  for (unsigned q = 0u; q < 2u; ++q) {
-    const unsigned o = (x0 + 2u * q) & 63u;
-    Yb[q] = *reinterpret_cast<const double2 *>(yp + o);
+    for (unsigned v = 0u; v < YU; ++v)
+      Yb[q][v] = *reinterpret_cast<const double2 *>(yp + v * dy * kGramColLd + o);
 #pragma unroll
-    for (unsigned u = 0u; u < 4u; ++u)
-      Xb[q][u] = *reinterpret_cast<const double2 *>(xp + u * kGramColLd + o);
-  }
+    for (unsigned u = 0u; u < XU; ++u)
+      if (LX > 1u || (2u * kp + 1u >= u && 2u * kp <= u + 63u))
+        Xb[q][u] = *reinterpret_cast<const double2 *>(xp + u * kGramColLd + o);
+  };
+  load(0u);
+  load(1u);
 #pragma unroll
-  for (unsigned kp = 0u; kp < 34u; ++kp) { // pairs k = 2kp, 2kp + 1
-    if (kp + 2u < 34u) {
-      const unsigned q = (kp + 2u) % 3u;
-      const unsigned o = (x0 + 2u * (kp + 2u)) & 63u;
-      Yb[q] = *reinterpret_cast<const double2 *>(yp + o);
-#pragma unroll
-      for (unsigned u = 0u; u < 4u; ++u)
-        if (2u * (kp + 2u) + 1u >= u && 2u * (kp + 2u) <= u + 63u)
-          Xb[q][u] = *reinterpret_cast<const double2 *>(xp + u * kGramColLd + o);
-    }
-    const unsigned q = kp % 3u;
-#pragma unroll
-    for (unsigned h = 0u; h < 2u; ++h) {
-      const unsigned k = 2u * kp + h;
-      const double yv = h ? Yb[q].y : Yb[q].x;
-#pragma unroll
-      for (unsigned u = 0u; u < 4u; ++u)
-        if (k >= u && k <= u + 63u)
-          acc[u] = __fma_rn(yv, h ? Xb[q][u].y : Xb[q][u].x, acc[u]);
-    }
-  }
-}
-
-// The same for the 8 chains (x0+u, y0) and (x0+u, y1) of a lane (one CTA per
-// block pair): both columns share the diagonal operands, so each 16-byte
-// diagonal load feeds 4 FMAs instead of 2.
-__device__ __forceinline__ void gram_tile2(const double *const st, const unsigned base, const unsigned x0,
-                                           const unsigned y0, const unsigned y1, double (&acc)[4][2])
-{
-  const double *const yp0 = st + base + y0 * kGramColLd;
-  const double *const yp1 = st + base + y1 * kGramColLd;
-  const double *const xp = st + base + x0 * kGramColLd;
-  double2 Yb[3][2], Xb[3][4];
-#pragma unroll
-  for (unsigned q = 0u; q < 2u; ++q) {
-    const unsigned o = (x0 + 2u * q) & 63u;
-    Yb[q][0] = *reinterpret_cast<const double2 *>(yp0 + o);
-    Yb[q][1] = *reinterpret_cast<const double2 *>(yp1 + o);
-#pragma unroll
-    for (unsigned u = 0u; u < 4u; ++u)
-      Xb[q][u] = *reinterpret_cast<const double2 *>(xp + u * kGramColLd + o);
-  }
-#pragma unroll
-  for (unsigned kp = 0u; kp < 34u; ++kp) { // pairs k = 2kp, 2kp + 1
-    if (kp + 2u < 34u) {
-      const unsigned q = (kp + 2u) % 3u;
-      const unsigned o = (x0 + 2u * (kp + 2u)) & 63u;
-      Yb[q][0] = *reinterpret_cast<const double2 *>(yp0 + o);
-      Yb[q][1] = *reinterpret_cast<const double2 *>(yp1 + o);
-#pragma unroll
-      for (unsigned u = 0u; u < 4u; ++u)
-        if (2u * (kp + 2u) + 1u >= u && 2u * (kp + 2u) <= u + 63u)
-          Xb[q][u] = *reinterpret_cast<const double2 *>(xp + u * kGramColLd + o);
-    }
+  for (unsigned kp = 0u; kp < NP; ++kp) { // pairs k = 2kp, 2kp + 1
+    if (kp + 2u < NP)
+      load(kp + 2u);
     const unsigned q = kp % 3u;
 #pragma unroll
     for (unsigned h = 0u; h < 2u; ++h) {
       const unsigned k = 2u * kp + h;
 #pragma unroll
-      for (unsigned v = 0u; v < 2u; ++v) {
-        const double yv = h ? Yb[q][v].y : Yb[q][v].x;
+      for (unsigned u = 0u; u < XU; ++u) {
+        const double xv = h ? Xb[q][u].y : Xb[q][u].x;
+        if (k < u || k > (LX - 1u) * XU + u + 63u) // no lane's row
+          continue;
+        // lx = 0 has begun at k = u and ends at u + 63, lx = 1 XU later
+        const bool on = (LX == 1u) ? true : (k < XU + u) ? (lx == 0u) : (k > u + 63u) ? (lx != 0u) : true;
+        if (on) {
 #pragma unroll
-        for (unsigned u = 0u; u < 4u; ++u)
-          if (k >= u && k <= u + 63u)
-            acc[u][v] = __fma_rn(yv, h ? Xb[q][u].y : Xb[q][u].x, acc[u][v]);
+          for (unsigned v = 0u; v < YU; ++v)
+            acc[u][v] = __fma_rn(h ? Yb[q][v].y : Yb[q][v].x, xv, acc[u][v]);
+        }
       }
     }
   }
 }
 
-// Lanes of gram_tile2 (one CTA per pair): x-block b (rows 4b..4b+3) has
-// 2(b+1) lanes; its lane j takes columns y0 = j and y1 = j + 2(b+1), i.e. all
-// y = 0..4b+3 (entries with y > x are computed and dropped).  72 lanes in 3
-// warps: x-blocks (7, 6, 0), (5, 4, 3), (2, 1).
-__device__ __forceinline__ bool gram_lane2(const unsigned warp, const unsigned lane, unsigned &x0, unsigned &y0,
-                                           unsigned &y1)
+// The lanes.  x-block b is the rows LX XU b .. LX XU (b + 1) - 1.  It has the
+// columns y = 0 .. LX XU (b + 1) - 1 (entries with y > x are computed and
+// dropped), nj = LX XU (b + 1) / YU of them with v = 0; its lane LX j + lx takes
+// y = j + v nj.  Blocks of the warps:
+//   1 CTA: 4x2, LX 1; warps (7, 6, 0), (5, 4, 3), (2, 1): 72 lanes.
+//   2 CTAs: 2x2, LX 2; (7), (6, 0), (1) of rank 0, (5), (4, 2), (3) of rank 1:
+//     72 lanes.
+//   4 CTAs: 1x2, LX 2; (15 - rank), (8 + rank, rank), (7 - rank): 68 lanes.
+//   8 CTAs: 1x1, LX 2; block 15 - rank in warps 0 and 1, block rank in warp 2:
+//     68 lanes.
+template <unsigned NSPLIT> struct GramShape {
+  static constexpr unsigned XU = (NSPLIT == 1u) ? 4u : (NSPLIT == 2u) ? 2u : 1u;
+  static constexpr unsigned YU = (NSPLIT <= 4u) ? 2u : 1u;
+  static constexpr unsigned LX = (NSPLIT == 1u) ? 1u : 2u;
+  static constexpr unsigned warps = 3u;
+};
+
+struct GramLane {
+  unsigned X0, lx, y0, dy;
+  bool on;
+};
+
+template <unsigned NSPLIT>
+__device__ __forceinline__ GramLane gram_lane(const unsigned rank, const unsigned warp, const unsigned lane)
 {
-  if (warp >= 3u)
-    return false;
-  unsigned first = 0u;
+  using S = GramShape<NSPLIT>;
+  GramLane g = {0u, 0u, 0u, 0u, false};
+  if (warp >= S::warps)
+    return g;
+  int blk[3] = {-1, -1, -1}; // the warp's blocks, in the order of their lanes
+  unsigned l = lane;
+  if constexpr (NSPLIT == 1u) {
+    blk[0] = (warp == 0u) ? 7 : (warp == 1u) ? 5 : 2;
+    blk[1] = (warp == 0u) ? 6 : (warp == 1u) ? 4 : 1;
+    blk[2] = (warp == 0u) ? 0 : (warp == 1u) ? 3 : -1;
+  }
+  else if constexpr (NSPLIT == 2u) {
+    blk[0] = (rank == 0u) ? ((warp == 2u) ? 1 : 7 - (int)warp) : 5 - (int)warp;
+    blk[1] = (warp == 1u) ? (rank == 0u ? 0 : 2) : -1;
+  }
+  else if constexpr (NSPLIT == 4u) {
+    blk[0] = (warp == 0u) ? 15 - (int)rank : (warp == 1u) ? 8 + (int)rank : 7 - (int)rank;
+    blk[1] = (warp == 1u) ? (int)rank : -1;
+  }
+  else {
+    blk[0] = (warp < 2u) ? 15 - (int)rank : (int)rank;
+    l = (warp == 1u) ? lane + 32u : lane;
+  }
 #pragma unroll
   for (unsigned i = 0u; i < 3u; ++i) {
-    const int b = (warp == 0u) ? ((i == 0u) ? 7 : (i == 1u) ? 6 : 0)
-                               : (warp == 1u) ? ((i == 0u) ? 5 : (i == 1u) ? 4 : 3) : ((i == 0u) ? 2 : (i == 1u) ? 1 : -1);
-    if (b < 0)
-      return false;
-    const unsigned nl = 2u * (unsigned)b + 2u;
-    if (lane < first + nl) {
-      const unsigned j = lane - first;
-      x0 = 4u * (unsigned)b;
-      y0 = j;
-      y1 = j + nl;
-      return true;
+    if (blk[i] < 0)
+      return g;
+    const unsigned b = (unsigned)blk[i], nj = S::LX * S::XU * (b + 1u) / S::YU;
+    if (l < S::LX * nj) {
+      g.X0 = S::LX * S::XU * b;
+      g.lx = l % S::LX;
+      g.y0 = l / S::LX;
+      g.dy = nj;
+      g.on = true;
+      return g;
     }
-    first += nl;
+    l -= S::LX * nj;
   }
-  return false;
+  return g;
 }
 
-// The 2 chains (x0, y) and (x0+1, y) of a lane, in acc[0] and acc[1]
-// (4-CTA clusters: each CTA has a quarter of the entries, and thinner lane
-// tiles give it 3 warps): chain u takes the k in [u, u+63], so 33 row pairs.
-__device__ __forceinline__ void gram_tile_n2(const double *const st, const unsigned base, const unsigned x0,
-                                             const unsigned y, double (&acc)[4])
-{
-  const double *const yp = st + base + y * kGramColLd;
-  const double *const xp = st + base + x0 * kGramColLd;
-  double2 Yb[3], Xb[3][2];
+// a lane's chains
+template <unsigned NSPLIT> struct GramAcc {
+  using S = GramShape<NSPLIT>;
+  double a[S::XU][S::YU];
+  __device__ __forceinline__ void clear()
+  {
 #pragma unroll
-  for (unsigned q = 0u; q < 2u; ++q) {
-    const unsigned o = (x0 + 2u * q) & 63u;
-    Yb[q] = *reinterpret_cast<const double2 *>(yp + o);
+    for (unsigned u = 0u; u < S::XU; ++u)
 #pragma unroll
-    for (unsigned u = 0u; u < 2u; ++u)
-      Xb[q][u] = *reinterpret_cast<const double2 *>(xp + u * kGramColLd + o);
+      for (unsigned v = 0u; v < S::YU; ++v)
+        a[u][v] = +0.0;
   }
-#pragma unroll
-  for (unsigned kp = 0u; kp < 33u; ++kp) { // pairs k = 2kp, 2kp + 1
-    if (kp + 2u < 33u) {
-      const unsigned q = (kp + 2u) % 3u;
-      const unsigned o = (x0 + 2u * (kp + 2u)) & 63u;
-      Yb[q] = *reinterpret_cast<const double2 *>(yp + o);
-#pragma unroll
-      for (unsigned u = 0u; u < 2u; ++u)
-        if (2u * (kp + 2u) + 1u >= u && 2u * (kp + 2u) <= u + 63u)
-          Xb[q][u] = *reinterpret_cast<const double2 *>(xp + u * kGramColLd + o);
-    }
-    const unsigned q = kp % 3u;
-#pragma unroll
-    for (unsigned h = 0u; h < 2u; ++h) {
-      const unsigned k = 2u * kp + h;
-      const double yv = h ? Yb[q].y : Yb[q].x;
-#pragma unroll
-      for (unsigned u = 0u; u < 2u; ++u)
-        if (k >= u && k <= u + 63u)
-          acc[u] = __fma_rn(yv, h ? Xb[q][u].y : Xb[q][u].x, acc[u]);
-    }
+  __device__ __forceinline__ void tile(const double *const st, const GramLane &g)
+  {
+    gram_tile<S::XU, S::YU, S::LX>(st, g.X0, g.lx, g.y0, g.dy, a);
   }
-}
-
-// Lanes of gram_tile_n2 in a 4-CTA cluster: x-block b (rows 2b, 2b+1) has the
-// lanes y = 0..2b+1 (entries with y > x are computed and dropped); CTA r
-// takes x-blocks 15-r (warp 0), 8+r then r (warp 1) and 7-r (warp 2): 68
-// lanes in every CTA.
-__device__ __forceinline__ bool gram_lane_q(const unsigned rank, const unsigned warp, const unsigned lane,
-                                            unsigned &x0, unsigned &y)
-{
-  unsigned b, first = 0u;
-  if (warp == 0u)
-    b = 15u - rank;
-  else if (warp == 1u) {
-    const unsigned n1 = 2u * (8u + rank) + 2u;
-    b = (lane < n1) ? 8u + rank : rank;
-    first = (lane < n1) ? 0u : n1;
+  // the entries of the lower triangle: put(offset y * 32 + x, value)
+  template <typename F> __device__ __forceinline__ void put(const GramLane &g, const F &f) const
+  {
+    if (!g.on)
+      return;
+    const unsigned x0 = g.X0 + g.lx * S::XU;
+#pragma unroll
+    for (unsigned u = 0u; u < S::XU; ++u)
+#pragma unroll
+      for (unsigned v = 0u; v < S::YU; ++v) {
+        const unsigned y = g.y0 + v * g.dy;
+        if (x0 + u >= y)
+          f(y * 32u + x0 + u, a[u][v]);
+      }
   }
-  else if (warp == 2u)
-    b = 7u - rank;
-  else
-    return false;
-  if (lane >= first + 2u * b + 2u)
-    return false;
-  x0 = 2u * b;
-  y = lane - first;
-  return true;
-}
-
-// Lanes of gram_tile (2-CTA clusters): x-block xb (rows 4xb..4xb+3)
-// has the lanes y = 0..4xb+3 (entries with y > x are computed and dropped).
-// A warp takes a primary x-block p (lanes 0..4p+3) and possibly a secondary
-// one s (the next 4s+4 lanes), so that the 4 operands of column x0+u are
-// shared by the warp.
-//   rank 0: (7), (6,0), (1); rank 1: (5), (4,2), (3)
-template <unsigned NSPLIT>
-__device__ __forceinline__ bool gram_lane_of(const unsigned rank, const unsigned warp, const unsigned lane,
-                                             unsigned &x0, unsigned &y)
-{
-  static_assert(NSPLIT == 2u, "the lane map of 2-CTA clusters");
-  if (warp >= 3u) // rank 0: (7), (6,0), (1); rank 1: (5), (4,2), (3)
-    return false;
-  const int p = (rank == 0u) ? ((warp == 2u) ? 1 : 7 - (int)warp) : 5 - (int)warp;
-  const int sb = (warp == 1u) ? (rank == 0u ? 0 : 2) : -1;
-  const unsigned np = 4u * (unsigned)p + 4u;
-  if (lane < np) {
-    x0 = 4u * (unsigned)p;
-    y = lane;
-    return true;
-  }
-  if (sb >= 0 && lane < np + 4u * (unsigned)sb + 4u) {
-    x0 = 4u * (unsigned)sb;
-    y = lane - np;
-    return true;
-  }
-  return false;
-}
+};
 
 // ---------------------------------------------------------------------------
 // Right-looking Cholesky of the lower triangle held in R, by one warp with
@@ -939,19 +881,9 @@ __device__ __forceinline__ void pair_step(const StepParams &P, const unsigned st
   else {
   // ------------------------------ 1. Gram --------------------------------
   const unsigned ntile = P.nrow >> 6; // 64-row tiles
-  // chains per lane: 8 with one CTA per pair (gram_tile2), 4 with 2 CTAs
-  // (gram_tile), 2 with 4 CTAs (gram_tile_n2); 3 Gram warps each
-  unsigned gx0 = 0u, gy = 0u, gy1 = 0u;
-  const unsigned gwarps = 3u;
-  bool gthr;
-  if constexpr (NSPLIT == 1u)
-    gthr = gram_lane2(warp, lane, gx0, gy, gy1);
-  else if constexpr (NSPLIT == 4u)
-    gthr = gram_lane_q(rank, warp, lane, gx0, gy);
-  else
-    gthr = gram_lane_of<NSPLIT>(rank, warp, lane, gx0, gy);
-  double gacc[4] = {+0.0, +0.0, +0.0, +0.0};
-  double gacc2[4][2] = {{+0.0, +0.0}, {+0.0, +0.0}, {+0.0, +0.0}, {+0.0, +0.0}};
+  const GramLane gl = gram_lane<NSPLIT>(rank, warp, lane);
+  GramAcc<NSPLIT> gacc;
+  gacc.clear();
 
   const unsigned ngst = (ntile + kGramTiles - 1u) / kGramTiles; // stages of 2 tiles
   // thread 0: the TMA engine brings stage k, per tile block i's and block j's
@@ -976,19 +908,13 @@ __device__ __forceinline__ void pair_step(const StepParams &P, const unsigned st
     if (tid == kIssuer && k + kGramStages - 1u < ngst)
       issue_gram(k + kGramStages - 1u); // into the buffer released at the end of stage k - 1
     int fail = 0;
-    if (warp < gwarps) {
+    if (warp < GramShape<NSPLIT>::warps) {
       if (!mbar_wait_bounded(&bars[k % kGramStages], (k / kGramStages) & 1u, kWaitLimit))
         fail = 1;
-      else if (gthr) {
+      else if (gl.on) {
         const unsigned nt = min(kGramTiles, ntile - k * kGramTiles);
-        for (unsigned t = 0u; t < nt; ++t) {
-          if constexpr (NSPLIT == 1u)
-            gram_tile2(stg + (k % kGramStages) * kGramStage, t * kGramTileLd, gx0, gy, gy1, gacc2);
-          else if constexpr (NSPLIT == 4u)
-            gram_tile_n2(stg + (k % kGramStages) * kGramStage, t * kGramTileLd, gx0, gy, gacc);
-          else
-            gram_tile(stg + (k % kGramStages) * kGramStage, t * kGramTileLd, gx0, gy, gacc);
-        }
+        for (unsigned t = 0u; t < nt; ++t)
+          gacc.tile(stg + (k % kGramStages) * kGramStage + t * kGramTileLd, gl);
       }
     }
     failed = __syncthreads_or(fail); // uniform decision
@@ -1001,31 +927,14 @@ __device__ __forceinline__ void pair_step(const StepParams &P, const unsigned st
     atomicOr(P.err, kErrWaitTimeout);
   }
   // our share of the lower triangle, into our R and the other CTAs' R
-  if constexpr (NSPLIT == 1u) {
-    if (gthr) {
+  {
+    cg::cluster_group cl = cg::this_cluster();
+    gacc.put(gl, [&](const unsigned o, const double v) {
+      R[o] = v;
 #pragma unroll
-      for (unsigned u = 0u; u < 4u; ++u)
-#pragma unroll
-        for (unsigned v = 0u; v < 2u; ++v) {
-          const unsigned y = v ? gy1 : gy;
-          if (gx0 + u >= y)
-            R[y * 32u + gx0 + u] = gacc2[u][v];
-        }
-    }
-  }
-  else if (gthr) {
-#pragma unroll
-    for (unsigned u = 0u; u < ((NSPLIT == 4u) ? 2u : 4u); ++u)
-      if (gx0 + u >= gy) {
-        const unsigned o = gy * 32u + gx0 + u;
-        R[o] = gacc[u];
-        if (NSPLIT > 1u) {
-          cg::cluster_group cl = cg::this_cluster();
-#pragma unroll
-          for (unsigned q = 1u; q < NSPLIT; ++q)
-            cl.map_shared_rank(R, (rank + q) % NSPLIT)[o] = gacc[u];
-        }
-      }
+      for (unsigned q = 1u; q < NSPLIT; ++q)
+        cl.map_shared_rank(R, (rank + q) % NSPLIT)[o] = v;
+    });
   }
   }
   if (NSPLIT > 1u)
@@ -1187,9 +1096,9 @@ __device__ __forceinline__ void pair_step2(const StepParams &PA, const unsigned 
   const unsigned ntA = PA.nrow >> 6, ntB = PB.nrow >> 6;
   const unsigned ngA = (ntA + kGramTiles - 1u) / kGramTiles, ngB = (ntB + kGramTiles - 1u) / kGramTiles;
   const unsigned ng = ngA + ngB;
-  unsigned gx0 = 0u, gy = 0u, gy1 = 0u;
-  const bool gthr = gram_lane2(warp, lane, gx0, gy, gy1);
-  double gacc[4][2] = {{+0.0, +0.0}, {+0.0, +0.0}, {+0.0, +0.0}, {+0.0, +0.0}};
+  const GramLane gl = gram_lane<1u>(0u, warp, lane);
+  GramAcc<1u> gacc;
+  gacc.clear();
   auto stage_tiles = [&](const unsigned k) {
     return (k < ngA) ? min(kGramTiles, ntA - k * kGramTiles) : min(kGramTiles, ntB - (k - ngA) * kGramTiles);
   };
@@ -1206,18 +1115,9 @@ __device__ __forceinline__ void pair_step2(const StepParams &PA, const unsigned 
       tma_load_3d(st + t * kGramTileLd + 16u * kGramColLd, tm, 0, (int)(t0 + t), cj, &bars[s]);
     }
   };
-  auto put_gram = [&](double *const R) { // our share of the lower triangle
-    if (gthr) {
-#pragma unroll
-      for (unsigned u = 0u; u < 4u; ++u)
-#pragma unroll
-        for (unsigned v = 0u; v < 2u; ++v) {
-          const unsigned y = v ? gy1 : gy;
-          if (gx0 + u >= y)
-            R[y * 32u + gx0 + u] = gacc[u][v];
-          gacc[u][v] = +0.0;
-        }
-    }
+  auto put_gram = [&](double *const R) { // the lower triangle
+    gacc.put(gl, [&](const unsigned o, const double v) { R[o] = v; });
+    gacc.clear();
   };
 
   if (tid == kIssuer)
@@ -1229,13 +1129,13 @@ __device__ __forceinline__ void pair_step2(const StepParams &PA, const unsigned 
     if (tid == kIssuer && k + kGramStages - 1u < ng)
       issue_gram(k + kGramStages - 1u);
     int fail = 0;
-    if (warp < 3u) {
+    if (warp < GramShape<1u>::warps) {
       if (!mbar_wait_bounded(&bars[k % kGramStages], (k / kGramStages) & 1u, kWaitLimit))
         fail = 1;
-      else if (gthr) {
+      else if (gl.on) {
         const unsigned nt = stage_tiles(k);
         for (unsigned t = 0u; t < nt; ++t)
-          gram_tile2(stg + (k % kGramStages) * kGramStage, t * kGramTileLd, gx0, gy, gy1, gacc);
+          gacc.tile(stg + (k % kGramStages) * kGramStage + t * kGramTileLd, gl);
       }
       if (k + 1u == ngA)
         put_gram(sm + kOffR);
@@ -1397,7 +1297,7 @@ __device__ __forceinline__ unsigned ld_acquire(const unsigned *p)
 // ---------------------------------------------------------------------------
 // One block pair on a CTA of 4 warps (batched form, two such CTAs per SM).
 // The arithmetic is that of pair_step with one CTA per pair -- the Gram
-// chains of gram_tile2 on warps 0-2 (warp 3 issues the tile copies), the
+// chains of pair_step with one CTA per pair on warps 0-2 (warp 3 issues the tile copies), the
 // Cholesky factorisation and quarter-warp inner sweeps of pair_step2's warp
 // groups, pair_step's update tiles (warp w takes row groups w and w + 4 of
 // every stage) -- so every matrix gets the bits of its single call.  Shared
@@ -1446,9 +1346,9 @@ __device__ __forceinline__ void pair_step_n(const StepParams &P, const unsigned 
 
   // ------------------------------ 1. Gram --------------------------------
   const unsigned ntile = P.nrow >> 6;
-  unsigned gx0 = 0u, gy = 0u, gy1 = 0u;
-  const bool gthr = gram_lane2(warp, lane, gx0, gy, gy1);
-  double gacc[4][2] = {{+0.0, +0.0}, {+0.0, +0.0}, {+0.0, +0.0}, {+0.0, +0.0}};
+  const GramLane gl = gram_lane<1u>(0u, warp, lane);
+  GramAcc<1u> gacc;
+  gacc.clear();
   auto issue_gram = [&](const unsigned k) { // tile k into stage k mod 4
     const unsigned s = k % kNGStages;
     double *const st = stg + s * kGramTileLd;
@@ -1465,11 +1365,11 @@ __device__ __forceinline__ void pair_step_n(const StepParams &P, const unsigned 
     if (tid == kNIssuer && k + kNGStages - 1u < ntile)
       issue_gram(k + kNGStages - 1u); // into the stage released after tile k - 1
     int fail = 0;
-    if (warp < 3u) {
+    if (warp < GramShape<1u>::warps) {
       if (!mbar_wait_bounded(&bars[k % kNGStages], (k / kNGStages) & 1u, kWaitLimit))
         fail = 1;
-      else if (gthr)
-        gram_tile2(stg + (k % kNGStages) * kGramTileLd, 0u, gx0, gy, gy1, gacc);
+      else if (gl.on)
+        gacc.tile(stg + (k % kNGStages) * kGramTileLd, gl);
     }
     failed = __syncthreads_or(fail);
     if (failed)
@@ -1483,16 +1383,7 @@ __device__ __forceinline__ void pair_step_n(const StepParams &P, const unsigned 
     }
     return;
   }
-  if (gthr) {
-#pragma unroll
-    for (unsigned u = 0u; u < 4u; ++u)
-#pragma unroll
-      for (unsigned v = 0u; v < 2u; ++v) {
-        const unsigned y = v ? gy1 : gy;
-        if (gx0 + u >= y)
-          R[y * 32u + gx0 + u] = gacc[u][v];
-      }
-  }
+  gacc.put(gl, [&](const unsigned o, const double v) { R[o] = v; });
   __syncthreads();
 
   // the first update stage: its rows do not change before the update, so the
@@ -1576,7 +1467,7 @@ __device__ __forceinline__ void pair_step_n(const StepParams &P, const unsigned 
 // ---------------------------------------------------------------------------
 // Two block pairs on a CTA of 4 warps (batched form, two such CTAs per SM:
 // four pairs in flight per SM).  Pair A of matrix PA, pair B of matrix PB:
-// their Grams (gram_tile2 on warps 0-2, copies by warp 3) and updates (warp w
+// their Grams (warps 0-2, copies by warp 3) and updates (warp w
 // takes row groups w and w + 4 of every stage) run on the 4 warps, A's then
 // B's, as one stream of tiles and one of stages; their Cholesky
 // factorisations and inner sweeps run concurrently, warps 0-1 on A (named
@@ -1625,9 +1516,9 @@ __device__ __forceinline__ void pair_step2n(const StepParams &PA, const unsigned
   // ------------------------------ 1. Grams --------------------------------
   // tiles 0 .. ntA-1 are A's, ntA .. ntA+ntB-1 B's
   const unsigned ntA = PA.nrow >> 6, ntB = PB.nrow >> 6, nt = ntA + ntB;
-  unsigned gx0 = 0u, gy = 0u, gy1 = 0u;
-  const bool gthr = gram_lane2(warp, lane, gx0, gy, gy1);
-  double gacc[4][2] = {{+0.0, +0.0}, {+0.0, +0.0}, {+0.0, +0.0}, {+0.0, +0.0}};
+  const GramLane gl = gram_lane<1u>(0u, warp, lane);
+  GramAcc<1u> gacc;
+  gacc.clear();
   auto issue_gram = [&](const unsigned k) {
     const unsigned s = k % kNGStages;
     const bool a = k < ntA;
@@ -1638,18 +1529,9 @@ __device__ __forceinline__ void pair_step2n(const StepParams &PA, const unsigned
     tma_load_3d(st, tm, 0, tile, (int)((a ? iA : iB) * kNColB), &bars[s]);
     tma_load_3d(st + 16u * kGramColLd, tm, 0, tile, (int)((a ? jA : jB) * kNColB), &bars[s]);
   };
-  auto put_gram = [&](double *const R) { // our share of the lower triangle
-    if (gthr) {
-#pragma unroll
-      for (unsigned u = 0u; u < 4u; ++u)
-#pragma unroll
-        for (unsigned v = 0u; v < 2u; ++v) {
-          const unsigned y = v ? gy1 : gy;
-          if (gx0 + u >= y)
-            R[y * 32u + gx0 + u] = gacc[u][v];
-          gacc[u][v] = +0.0;
-        }
-    }
+  auto put_gram = [&](double *const R) { // the lower triangle
+    gacc.put(gl, [&](const unsigned o, const double v) { R[o] = v; });
+    gacc.clear();
   };
   if (tid == kNIssuer)
     for (unsigned k = 0u; k + 1u < kNGStages && k < nt; ++k)
@@ -1660,11 +1542,11 @@ __device__ __forceinline__ void pair_step2n(const StepParams &PA, const unsigned
     if (tid == kNIssuer && k + kNGStages - 1u < nt)
       issue_gram(k + kNGStages - 1u);
     int fail = 0;
-    if (warp < 3u) {
+    if (warp < GramShape<1u>::warps) {
       if (!mbar_wait_bounded(&bars[k % kNGStages], (k / kNGStages) & 1u, kWaitLimit))
         fail = 1;
-      else if (gthr)
-        gram_tile2(stg + (k % kNGStages) * kGramTileLd, 0u, gx0, gy, gy1, gacc);
+      else if (gl.on)
+        gacc.tile(stg + (k % kNGStages) * kGramTileLd, gl);
       if (k + 1u == ntA)
         put_gram(sm + kN2OffRA);
       else if (k + 1u == nt)

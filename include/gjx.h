@@ -103,8 +103,9 @@ int gjx_hypJacL2_batched(unsigned routine, unsigned nmat, const unsigned *nrow, 
  * the same bits either way. */
 void gjx_set_sweep_mode(int mode);
 
-/* CTAs per block pair (a thread-block cluster): 1, 2 or 4, or 0 (default)
- * for the automatic choice.  The results are the same bits for any value. */
+/* CTAs per block pair (a thread-block cluster): 1, 2, 4 or 8 (8: launches per
+ * step only), or 0 (default) for the automatic choice.  The results are the
+ * same bits for any value. */
 void gjx_set_split(unsigned n);
 
 /* Block pairs that a CTA takes at a time: 2 (the Cholesky factorisations
@@ -132,7 +133,7 @@ void gjx_set_pairs_per_cta(unsigned w);
 void gjx_set_variant(unsigned v);
 
 /*
- * Autotuner: time every launch configuration of this shape -- 1, 2 or 4
+ * Autotuner: time every launch configuration of this shape -- 1, 2, 4 or 8
  * CTAs per block pair (where the pairs fit), one launch per outer step or
  * per sweep -- on a seeded random nrow x ncol matrix in scratch device
  * memory, `sweeps` outer sweeps each (0: 1), and use the fastest in later
