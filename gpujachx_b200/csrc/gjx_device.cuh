@@ -484,6 +484,14 @@ __device__ __forceinline__ void tma_store_3d(const CUtensorMap *tm, const void *
                : "memory");
 }
 
+// 1-D bulk copy shared -> global in this thread's current bulk async-group;
+// dst, src 16-byte aligned, bytes a multiple of 16
+__device__ __forceinline__ void bulk_s2g(void *dst, const void *src, const uint32_t bytes)
+{
+  asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst), "r"(smem_u32(src)), "r"(bytes)
+               : "memory");
+}
+
 // close this thread's bulk async-group
 __device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
 

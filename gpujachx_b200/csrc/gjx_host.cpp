@@ -45,6 +45,8 @@ struct Strat {
   std::string sdy, snp0, snp1; // where other tables of the families come from (batched and split forms)
 };
 
+constexpr unsigned kUpdateMargin = 1u; // stages of 256 rows
+
 std::mutex g_mtx;
 Strat g_strat;
 int g_verbose = 1;
@@ -117,6 +119,8 @@ struct DevCtx {
   unsigned long long *d_cnt = nullptr; // [0] = cvg, [1] = err (int in the low word)
   unsigned long long *h_cnt = nullptr; // pinned mirror
   unsigned *d_ver = nullptr;           // per-block write counts of the one-launch sweep (1024 blocks)
+  double *d_vt = nullptr;              // the transforms of a step and their flags (l1_update_kernel)
+  size_t vt_pairs = 0u;
   // outer tables of the batched form, by n1, for strategy version btab_version
   bool batch_ready = false;
   cudaStream_t batch_stream = nullptr; // graphs cannot be captured on the legacy default stream
@@ -181,6 +185,21 @@ int upload_strat(DevCtx &ctx, const cudaStream_t st)
   return 0;
 }
 
+// the transforms of a step of the loaded outer table (and their flags)
+int ensure_vt(DevCtx &ctx)
+{
+  const size_t pairs = g_strat.pairs1;
+  if (pairs <= ctx.vt_pairs)
+    return 0;
+  if (ctx.d_vt)
+    GJX_CUDA(cudaFree(ctx.d_vt), "cudaFree(transforms)");
+  ctx.d_vt = nullptr;
+  ctx.vt_pairs = 0u;
+  GJX_CUDA(cudaMalloc(&ctx.d_vt, pairs * (gjx::kTransform * sizeof(double) + sizeof(unsigned))), "cudaMalloc(transforms)");
+  ctx.vt_pairs = pairs;
+  return 0;
+}
+
 double secs(const clk::time_point a, const clk::time_point b)
 {
   return std::chrono::duration<double>(b - a).count();
@@ -191,13 +210,14 @@ double secs(const clk::time_point a, const clk::time_point b)
 // configured the kernels on this device and provides the device-side
 // working memory: the strategy tables d_s0 / d_s1 (uploaded) and two
 // 64-bit words d_cnt (counter, error word), plus a host mirror h_cnt of
-// those two words.  Nothing is allocated here (profiling events aside,
+// those two words; d_ver (1024 words) and d_vt (ensure_vt), or null: no
+// launch per sweep, no update launches.  Nothing is allocated here (profiling events aside,
 // with prof).
 int run_sweeps_core(const unsigned routine, const unsigned nrow, const unsigned ncol, const unsigned nplus,
                     double *const dG, const unsigned lddG, double *const dV, const unsigned lddV, double *const dD,
                     const cudaStream_t st, const uint8_t *const d_s0, const uint16_t *const d_s1,
                     unsigned long long *const d_cnt, unsigned long long *const h_cnt, unsigned *const d_ver,
-                    const bool prof,
+                    double *const d_vt, const bool prof,
                     unsigned *const glbSwp, unsigned long long *const glb_s, unsigned long long *const glb_b)
 {
   const bool cdsort = (routine & GJX_CDSORT_1) != 0u, full = (routine & GJX_FULL_SVD) != 0u,
@@ -246,6 +266,7 @@ int run_sweeps_core(const unsigned routine, const unsigned nrow, const unsigned 
   GJX_CUDA(cudaGetDevice(&dev), "cudaGetDevice");
   GJX_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "SM count");
   p.width = (p.split == 1u && (g_pairs_per_cta == 2u || (!g_pairs_per_cta && p.pairs > (unsigned)sms))) ? 2u : 1u;
+  p.sms = (unsigned)sms;
   p.variant = g_variant;
   if (p.variant) { // the QR factors: one CTA per block pair, one launch per outer step
     p.split = 1u;
@@ -266,6 +287,24 @@ int run_sweeps_core(const unsigned routine, const unsigned nrow, const unsigned 
   p.ver = d_ver;
   // one launch per sweep when all clusters of a step are resident together
   bool one_launch = d_ver && mode > 0 && g_strat.n1 <= 1024u && gjx::sweep_kernel_fits(cdsort, full, p);
+  // the update as a launch of its own, its 256-row stages dealt out to all
+  // SMs: where that leaves an SM fewer stages than the step kernel does (its
+  // CTAs update their own pairs, and SMs without a pair idle), by a margin for
+  // the second launch and the transforms' way through memory.  ms per call with
+  // / without: 3072^2 (16 stages against 24) 323 / 372, 4864^2 without V (20
+  // against 38) 1187 / 1511, 16384x256 (4 against 9) 23.1 / 24.7; but 4096x2048
+  // (11 against 12) 146 / 141, HSVD 2048x1024 (3 against 3) 30.4 / 28.1
+  if (d_vt && !one_launch && !p.variant && !g_pairs_per_cta) {
+    const unsigned nst = (nrow + 255u) / 256u + (full ? (ncol + 255u) / 256u : 0u);
+    const unsigned own = (p.width == 2u) ? 2u * nst : (nst + p.split - 1u) / p.split;
+    const unsigned dealt = (p.pairs * nst + p.sms - 1u) / p.sms;
+    if (dealt + kUpdateMargin < own) {
+      p.vt = d_vt;
+      p.vflag = reinterpret_cast<unsigned *>(d_vt + (size_t)p.pairs * gjx::kTransform);
+      if (p.width == 2u)
+        p.width = gjx::kWidthHalf;
+    }
+  }
   const unsigned cap = g_sweep_cap ? g_sweep_cap : gjx::kNSweep;
   while (blk_swp < cap) {
     GJX_CUDA(cudaMemsetAsync(d_cnt, 0, sizeof(unsigned long long), st), "clear counter");
@@ -294,7 +333,7 @@ int run_sweeps_core(const unsigned routine, const unsigned nrow, const unsigned 
         if (prof)
           GJX_CUDA(cudaEventRecord(g_prof.ev[2u * stp + 1u], st), "cudaEventRecord");
       }
-      g_prof.launches += g_strat.steps1;
+      g_prof.launches += (p.vt ? 2u : 1u) * g_strat.steps1;
     }
     g_prof.l1_launches += g_strat.steps1;
     ++blk_swp;
@@ -347,8 +386,10 @@ int run_sweeps(const unsigned routine, const unsigned nrow, const unsigned ncol,
     return r;
   if (const int r = upload_strat(*ctx, st))
     return r;
+  if (const int r = ensure_vt(*ctx))
+    return r;
   return run_sweeps_core(routine, nrow, ncol, nplus, dG, lddG, dV, lddV, dD, st, ctx->d_s0, ctx->d_s1, ctx->d_cnt,
-                         ctx->h_cnt, ctx->d_ver, g_prof.on, glbSwp, glb_s, glb_b);
+                         ctx->h_cnt, ctx->d_ver, ctx->d_vt, g_prof.on, glbSwp, glb_s, glb_b);
 }
 
 // argument checks of 1/HypJacL2.cu:39-77, same codes in the same order
@@ -829,8 +870,8 @@ int noalloc_sweeps(const unsigned routine, const unsigned nrow, const unsigned n
   return run_sweeps_core(routine, nrow, ncol, nplus, dG, lddG, dV, lddV, dD, st,
                          reinterpret_cast<const uint8_t *>(base + kScrS0),
                          reinterpret_cast<const uint16_t *>(base + kScrS1),
-                         reinterpret_cast<unsigned long long *>(base + kScrCnt), h_cnt, nullptr, false, glbSwp, glb_s,
-                         glb_b);
+                         reinterpret_cast<unsigned long long *>(base + kScrCnt), h_cnt, nullptr, nullptr, false,
+                         glbSwp, glb_s, glb_b);
 }
 
 int family_tables(const unsigned n0, const unsigned n1, std::vector<uint8_t> &s0, unsigned &steps0,
@@ -1237,8 +1278,10 @@ int gjx_release_cache(void)
       GJX_CUDA(cudaFree(c.dV), "cudaFree");
     if (c.dD)
       GJX_CUDA(cudaFree(c.dD), "cudaFree");
-    c.dG = c.dV = c.dD = nullptr;
-    c.capG = c.capV = c.capD = 0u;
+    if (c.d_vt)
+      GJX_CUDA(cudaFree(c.d_vt), "cudaFree");
+    c.dG = c.dV = c.dD = c.d_vt = nullptr;
+    c.capG = c.capV = c.capD = c.vt_pairs = 0u;
   }
   return 0;
 }
@@ -1435,6 +1478,8 @@ int gjx_autotune(const unsigned routine, const unsigned nrow, const unsigned nco
     return r;
   if (const int r = upload_strat(*ctx, nullptr))
     return r;
+  if (const int r = ensure_vt(*ctx))
+    return r;
   const bool full = (routine & GJX_FULL_SVD) != 0u;
   const unsigned ld = nrow + (nrow & 1u);
   double *mem = nullptr;
@@ -1474,7 +1519,7 @@ int gjx_autotune(const unsigned routine, const unsigned nrow, const unsigned nco
           break;
         }
         rc = run_sweeps_core(routine, nrow, ncol, nplus, g, ld, full ? v : nullptr, ncol, d, nullptr, ctx->d_s0,
-                             ctx->d_s1, ctx->d_cnt, ctx->h_cnt, ctx->d_ver, false, &swp, &s_, &b_);
+                             ctx->d_s1, ctx->d_cnt, ctx->h_cnt, ctx->d_ver, ctx->d_vt, false, &swp, &s_, &b_);
         if (!rc && (cudaEventRecord(e1, nullptr) != cudaSuccess || cudaEventSynchronize(e1) != cudaSuccess ||
                     cudaEventElapsedTime(&ms, e0, e1) != cudaSuccess))
           rc = GJX_ERR_CUDA;

@@ -10,6 +10,7 @@
 namespace gjx {
 
 constexpr unsigned kNColB = 16u;  // columns per block (share/HypJacL.hpp:112-116)
+constexpr unsigned kTransform = 32u * 34u; // doubles of a pair's entry of StepParams::vt
 constexpr unsigned kNSweep = 30u; // outer and full-block inner sweep cap (share/HypJacL.hpp:7-9)
 
 // Everything one launch of the block-pair step needs.  One CTA per block pair
@@ -31,9 +32,13 @@ struct alignas(64) StepParams {
   unsigned nswp0;               // inner sweeps per block pair (1 or 30)
   int gdefinite;                // +1 J = I, -1 J = -I, 0 mixed signs
   unsigned split;               // CTAs per block pair (a cluster): 1, 2, 4 or 8
-  unsigned width;               // with split 1: block pairs per CTA, 1 or 2 (l1_step2_kernel)
+  unsigned width;               // with split 1: block pairs per CTA, 1 or 2 (l1_step2_kernel), or kWidthHalf (with vt)
   unsigned steps1;              // outer steps per sweep (persistent sweep kernel)
   unsigned *ver;                // per block: CTAs that have finished writing it this sweep
+  double *vt;                   // per pair [32][34]: the step's transforms, when the update is a launch of
+                                // its own (l1_update_kernel); null: the step kernel updates
+  unsigned *vflag;              // per pair: the transform is not the identity
+  unsigned sms;                 // SMs of the device (the grid of l1_update_kernel)
   unsigned variant;             // pivot-block factor: 0 Gram + Cholesky, 1 QR, 2 QR + Drmac's sweep
 };
 

@@ -32,6 +32,129 @@ __global__ void __launch_bounds__(kThreads, 1) l1_step2_kernel(const __grid_cons
     pair_step<SORT, ACCV, 1u>(P, P.step, a, 0u, sm);
 }
 
+// one launch per outer step, one block pair per CTA of 4 warps, two CTAs per
+// SM, up to its transform (P.vt): a step with more pairs than SMs
+template <bool SORT>
+__global__ void __launch_bounds__(kNThreads, 2) l1_stepn_kernel(const __grid_constant__ StepParams P)
+{
+  extern __shared__ __align__(128) double sm[];
+  pair_step_n<SORT, false>(P, P.step, blockIdx.x, sm);
+}
+
+// ---------------------------------------------------------------------------
+// The update of a step by itself: [G_i G_j] <- [G_i G_j] V_loc, and V likewise,
+// for all block pairs (P.vt, P.vflag).  The 256-row stages of all pairs, in
+// order, are dealt out evenly to one CTA per SM; a CTA takes a contiguous run,
+// so its transform changes rarely (two buffers, the next pair's loaded with
+// its first stage).  Stages as in pair_step with three buffers.
+// ---------------------------------------------------------------------------
+constexpr unsigned kUOffVT = 3u * kUpdStage;
+constexpr unsigned kUOffBar = kUOffVT + 2u * kTransform; // [0..2] stages, [3..4] transforms
+constexpr unsigned kUSmemDoubles = kUOffBar + 8u;
+static_assert(kUSmemDoubles * sizeof(double) <= 227u * 1024u, "three stages and two transforms must fit");
+
+template <bool ACCV>
+__global__ void __launch_bounds__(kThreads, 1) l1_update_kernel(const __grid_constant__ StepParams P)
+{
+  extern __shared__ __align__(128) double sm[];
+  uint64_t *const bars = reinterpret_cast<uint64_t *>(sm + kUOffBar);
+  const unsigned tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u;
+  const unsigned nG = (P.nrow + kUpdRows - 1u) / kUpdRows;
+  const unsigned nst = nG + (ACCV ? (P.ncol + kUpdRows - 1u) / kUpdRows : 0u);
+  const unsigned total = P.pairs * nst, per = total / gridDim.x, extra = total % gridDim.x;
+  const unsigned first = blockIdx.x * per + min(blockIdx.x, extra);
+  const unsigned end = first + per + (blockIdx.x < extra ? 1u : 0u);
+  // the first stage from i on whose pair changes
+  const auto live = [&](unsigned i) {
+    while (i < end && !P.vflag[i / nst])
+      i = (i / nst + 1u) * nst;
+    return min(i, end);
+  };
+  const auto stage_at = [&](const unsigned i, const CUtensorMap *&tm, int &piece, int &ci, int &cj) {
+    const unsigned pair = i / nst, k = i - pair * nst;
+    const size_t pidx = ((size_t)P.step * P.pairs + pair) * 2u;
+    tm = (k < nG) ? &P.tmG : &P.tmV;
+    piece = (int)((((k < nG) ? k : (k - nG)) * kUpdRows) >> 5);
+    ci = (int)(P.strat1[pidx] * kNColB);
+    cj = (int)(P.strat1[pidx + 1u] * kNColB);
+  };
+  const auto load = [&](const unsigned i, const unsigned n) { // one thread: stage i as the n-th, 2 tensor copies
+    const CUtensorMap *tm;
+    int piece, ci, cj;
+    stage_at(i, tm, piece, ci, cj);
+    double *const st = sm + (n % 3u) * kUpdStage;
+    mbar_arrive_expect_tx(&bars[n % 3u], 2u * kUpdBoxBytes);
+    tma_load_3d(st, tm, 0, piece, ci, &bars[n % 3u]);
+    tma_load_3d(st + 16u * kUpdColLd, tm, 0, piece, cj, &bars[n % 3u]);
+  };
+  const auto load_vt = [&](const unsigned pair, const unsigned m) { // one thread: the CTA's m-th transform
+    mbar_arrive_expect_tx(&bars[3u + (m & 1u)], kTransform * 8u);
+    bulk_g2s(sm + kUOffVT + (m & 1u) * kTransform, P.vt + (size_t)pair * kTransform, kTransform * 8u,
+             &bars[3u + (m & 1u)]);
+  };
+  unsigned i = live(first);
+  if (i >= end)
+    return;
+  if (tid == 0u) {
+    for (unsigned b = 0u; b < 5u; ++b)
+      mbar_init(&bars[b], 1u);
+    mbar_fence_init();
+    load_vt(i / nst, 0u);
+    load(i, 0u);
+  }
+  __syncthreads();
+  const unsigned sub = lane & 7u, cg8 = lane >> 3;
+  bool fresh = true; // the transform of this stage's pair has not been waited for
+  for (unsigned n = 0u, m = 0u; i < end; ++n) { // the n-th stage, with the m-th transform
+    const unsigned j = live(i + 1u);
+    const bool turn = j < end && j / nst != i / nst;
+    if (tid == 0u && j < end) {
+      bulk_wait_read_but1(); // the store of the stage before the last has read its buffer out
+      load(j, n + 1u);
+      if (turn) // every warp is past the transform before the last
+        load_vt(j / nst, m + 1u);
+    }
+    bool ok = !fresh || mbar_wait_bounded(&bars[3u + (m & 1u)], (m >> 1) & 1u, kWaitLimit);
+    ok = ok && mbar_wait_bounded(&bars[n % 3u], (n / 3u) & 1u, kWaitLimit);
+    const int fail = !__all_sync(0xffffffffu, ok);
+    double *const st = sm + (n % 3u) * kUpdStage;
+    if (!fail) {
+      double acc[4][8];
+      update_stage(st, sm + kUOffVT + (m & 1u) * kTransform, warp, sub, cg8, acc);
+      __syncwarp();
+      update_put(st, acc, warp, sub, cg8);
+      fence_async_shared();
+    }
+    if (__syncthreads_or(fail)) { // uniform decision; drain (bounded), report
+      if (tid == 0u) {
+        (void)mbar_wait_bounded(&bars[n % 3u], (n / 3u) & 1u, kWaitLimit / 8);
+        if (fresh)
+          (void)mbar_wait_bounded(&bars[3u + (m & 1u)], (m >> 1) & 1u, kWaitLimit / 8);
+        if (j < end)
+          (void)mbar_wait_bounded(&bars[(n + 1u) % 3u], ((n + 1u) / 3u) & 1u, kWaitLimit / 8);
+        if (turn)
+          (void)mbar_wait_bounded(&bars[3u + ((m + 1u) & 1u)], ((m + 1u) >> 1) & 1u, kWaitLimit / 8);
+        bulk_wait_all();
+        atomicOr(P.err, kErrWaitTimeout);
+      }
+      return;
+    }
+    if (tid == 0u) {
+      const CUtensorMap *tm;
+      int piece, ci, cj;
+      stage_at(i, tm, piece, ci, cj);
+      tma_store_3d(tm, st, 0, piece, ci);
+      tma_store_3d(tm, st + 16u * kUpdColLd, 0, piece, cj);
+      bulk_commit();
+    }
+    fresh = turn;
+    m += turn ? 1u : 0u;
+    i = j;
+  }
+  if (tid == 0u)
+    bulk_wait_all();
+}
+
 // the reference's alternative builds (P.variant: 1 -DUSE_QR, 2 -DUSE_DRMAC):
 // one CTA per block pair, the QR factor in place of the Gram and Cholesky
 template <bool SORT, bool ACCV, unsigned FAC>
@@ -261,6 +384,13 @@ cudaError_t l1_configure()
   if ((e = set_smem2<false, false>()) || (e = set_smem2<false, true>()) || (e = set_smem2<true, false>()) ||
       (e = set_smem2<true, true>()))
     return e;
+  const int bu = (int)(kUSmemDoubles * sizeof(double)), bn = (int)batchn_smem_bytes();
+  constexpr auto kSmem = cudaFuncAttributeMaxDynamicSharedMemorySize;
+  if ((e = cudaFuncSetAttribute(l1_update_kernel<false>, kSmem, bu)) ||
+      (e = cudaFuncSetAttribute(l1_update_kernel<true>, kSmem, bu)) ||
+      (e = cudaFuncSetAttribute(l1_stepn_kernel<false>, kSmem, bn)) ||
+      (e = cudaFuncSetAttribute(l1_stepn_kernel<true>, kSmem, bn)))
+    return e;
   const int b3 = (int)step_smem_bytes(2u);
   if ((e = set_smem<false, false, 1u>(b)) || (e = set_smem<false, true, 1u>(b)) || (e = set_smem<true, false, 1u>(b)) ||
       (e = set_smem<true, true, 1u>(b)) || (e = set_smem<false, false, 2u>(b3)) || (e = set_smem<false, true, 2u>(b3)) ||
@@ -429,6 +559,37 @@ template <bool S, bool A, unsigned F> static cudaError_t launch_var(const StepPa
   return cudaGetLastError();
 }
 
+// the block pairs of a step up to their transforms (p.vt), by the step kernels
+// without V (they leave before the update)
+static cudaError_t launch_factor(const bool sort, const StepParams &p, cudaStream_t s)
+{
+  if (p.width == kWidthHalf) {
+    if (sort)
+      l1_stepn_kernel<true><<<p.pairs, kNThreads, batchn_smem_bytes(), s>>>(p);
+    else
+      l1_stepn_kernel<false><<<p.pairs, kNThreads, batchn_smem_bytes(), s>>>(p);
+    return cudaGetLastError();
+  }
+  switch (p.split) {
+  case 8u:
+    return sort ? launch<true, false, 8u>(p, s) : launch<false, false, 8u>(p, s);
+  case 4u:
+    return sort ? launch<true, false, 4u>(p, s) : launch<false, false, 4u>(p, s);
+  case 2u:
+    return sort ? launch<true, false, 2u>(p, s) : launch<false, false, 2u>(p, s);
+  default:
+    return sort ? launch<true, false, 1u>(p, s) : launch<false, false, 1u>(p, s);
+  }
+}
+
+template <bool A> static cudaError_t launch_update(const StepParams &p, cudaStream_t s)
+{
+  const unsigned nst = (p.nrow + kUpdRows - 1u) / kUpdRows + (A ? (p.ncol + kUpdRows - 1u) / kUpdRows : 0u);
+  const unsigned total = p.pairs * nst;
+  l1_update_kernel<A><<<total < p.sms ? total : p.sms, kThreads, kUSmemDoubles * sizeof(double), s>>>(p);
+  return cudaGetLastError();
+}
+
 cudaError_t launch_l1_step(const bool sort, const bool accv, const StepParams &p, cudaStream_t s)
 {
   if (p.variant == 1u) {
@@ -440,6 +601,10 @@ cudaError_t launch_l1_step(const bool sort, const bool accv, const StepParams &p
     if (sort)
       return accv ? launch_var<true, true, 2u>(p, s) : launch_var<true, false, 2u>(p, s);
     return accv ? launch_var<false, true, 2u>(p, s) : launch_var<false, false, 2u>(p, s);
+  }
+  if (p.vt) {
+    const cudaError_t e = launch_factor(sort, p, s);
+    return (e != cudaSuccess) ? e : (accv ? launch_update<true>(p, s) : launch_update<false>(p, s));
   }
   const unsigned n = p.split;
   if (n == 1u && p.width == 2u) {

@@ -79,6 +79,7 @@ constexpr unsigned kUpdColLd = 272u;
 constexpr unsigned kUpdStages = 2u;
 constexpr unsigned kUpdStage = 32u * kUpdColLd; // doubles
 constexpr unsigned kVTLd = 34u;                 // B^T rows (V_loc transposed)
+static_assert(kTransform == 32u * kVTLd, "the layout of StepParams::vt");
 constexpr uint32_t kUpdBoxBytes = 34u * 8u * 16u * 8u;
 
 constexpr unsigned kRegion =
@@ -842,6 +843,27 @@ __device__ __forceinline__ void add_counts(const StepParams &P, const unsigned b
     atomicAdd(reinterpret_cast<unsigned *>(P.cvg), blk_s);
 }
 
+// V_loc of block pair `pair`, transposed as update_stage reads it, and whether
+// the pair changes, for l1_update_kernel (R is dead)
+template <unsigned THREADS>
+__device__ __forceinline__ void put_transform(const StepParams &P, const unsigned pair, const bool changes,
+                                              double *const R, const double *const Vl)
+{
+  const unsigned tid = threadIdx.x;
+  for (unsigned i = tid; i < 1024u; i += THREADS) {
+    const unsigned c = i >> 5, s = i & 31u;
+    R[s * kVTLd + c] = E32(Vl, s, c);
+  }
+  fence_async_shared();
+  __syncthreads();
+  if (tid == 0u) {
+    bulk_s2g(P.vt + (size_t)pair * kTransform, R, kTransform * 8u);
+    bulk_commit();
+    P.vflag[pair] = changes ? 1u : 0u;
+    bulk_wait_all();
+  }
+}
+
 // ---------------------------------------------------------------------------
 // The block-pair step kernel.
 // ---------------------------------------------------------------------------
@@ -961,7 +983,8 @@ __device__ __forceinline__ void pair_step(const StepParams &P, const unsigned st
     tma_load_3d(st, tm, 0, piece, (int)(iBlk * kNColB), &bars[4u + s]);
     tma_load_3d(st + 16u * kUpdColLd, tm, 0, piece, (int)(jBlk * kNColB), &bars[4u + s]);
   };
-  if (tid == 0u && nmine > 0u)
+  const bool apart = P.vt != nullptr; // the update is another kernel's (l1_update_kernel)
+  if (tid == 0u && nmine > 0u && !apart)
     issue_upd(0u);
 
   // ---------------------------- 2. Cholesky -------------------------------
@@ -983,6 +1006,11 @@ __device__ __forceinline__ void pair_step(const StepParams &P, const unsigned st
 
   if (rank == 0u && tid == 0u)
     add_counts(P, blk_s, blk_b);
+  if (apart) {
+    if (rank == 0u)
+      put_transform<kThreads>(P, pair, SORT || blk_s, R, Vl);
+    return;
+  }
   if (!SORT && !blk_s) { // no rotation: the block pair is unchanged
     if (tid == 0u && nmine > 0u && !mbar_wait_bounded(&bars[4u], 0u, kWaitLimit))
       atomicOr(P.err, kErrWaitTimeout); // the prefetched copy has landed before we leave
@@ -1398,7 +1426,8 @@ __device__ __forceinline__ void pair_step_n(const StepParams &P, const unsigned 
     tma_load_3d(stg, tm, 0, piece, (int)(iBlk * kNColB), &bars[4]);
     tma_load_3d(stg + 16u * kUpdColLd, tm, 0, piece, (int)(jBlk * kNColB), &bars[4]);
   };
-  if (tid == 0u && nst > 0u)
+  const bool apart = P.vt != nullptr; // the update is another kernel's (l1_update_kernel)
+  if (tid == 0u && nst > 0u && !apart)
     issue_upd(0u);
 
   // ------------------- 2.-3. Cholesky and inner sweeps --------------------
@@ -1414,6 +1443,10 @@ __device__ __forceinline__ void pair_step_n(const StepParams &P, const unsigned 
                        sm + kNOffRot + 16u * warp);
   if (tid == 0u)
     add_counts(P, blk_s, blk_b);
+  if (apart) {
+    put_transform<kNThreads>(P, pair, SORT || blk_s, R, Vl);
+    return;
+  }
   if (!SORT && !blk_s) { // no rotation: the block pair is unchanged
     if (tid == 0u && nst > 0u && !mbar_wait_bounded(&bars[4], 0u, kWaitLimit))
       atomicOr(P.err, kErrWaitTimeout); // the prefetched copy has landed before we leave

@@ -1,6 +1,9 @@
 """The routes of a single decomposition's outer steps against the fused step
 kernel with one CTA per block pair, which the other tests hold against the
-oracle: clusters of 2, 4 and 8 CTAs per pair.  The same bits."""
+oracle: clusters of 2, 4 and 8 CTAs per pair; the update as a launch of its
+own, its stages dealt out to all SMs, with 1 to 8 CTAs per pair before it, with
+more pairs than SMs, with partial stages and with pairs that do not change.
+The same bits."""
 
 import numpy as np
 import pytest
@@ -42,3 +45,33 @@ def test_clusters(m, n, nplus, alg, split, built):
     finally:
         g.lib().gjx_set_split(0)
         g.lib().gjx_set_sweep_mode(-1)
+
+
+@pytest.mark.parametrize("m,n,nplus,alg", [(6016, 640, 640, 11), (8256, 896, 300, 10), (3072, 2560, 2560, 9),
+                                           (3136, 3072, 1000, 11), (5120, 5120, 5120, 9)])
+def test_update_launch(m, n, nplus, alg, built):
+    import gpujachx_b200 as g
+    G = synth.make("gaussian", m, n, 6)
+    g.init_strats(None, "cycwor", 32, "cycwor", n // 16)
+    ref = _fused(g, alg, G, nplus)
+    g.lib().gjx_set_sweep_mode(-1)
+    g.profile(False)
+    r = g.hypJacL2(alg, G, nplus)
+    assert g.profile_read()["launches"] > 2 * (n // 16 - 1) * r.sweeps  # two launches a step
+    _same(r, ref, alg & 2)
+
+
+def test_update_launch_with_unchanged_pairs(built):
+    """Blocks orthogonal to each other, some of them orthogonal within: most
+    pairs keep their columns (ALG 10 does not sort)."""
+    import gpujachx_b200 as g
+    m, n = 8192, 640
+    r = np.random.default_rng(4)
+    G = np.zeros((m, n), order="F")
+    for b in range(n // 16):
+        blk = r.standard_normal((m // 64, 16))
+        G[b * (m // 64):(b + 1) * (m // 64), 16 * b:16 * b + 16] = blk if b % 5 == 0 else np.linalg.qr(blk)[0] * 2.0 ** (b % 7)
+    g.init_strats(None, "cycwor", 32, "cycwor", n // 16)
+    ref = _fused(g, 10, G, n)
+    g.lib().gjx_set_sweep_mode(-1)
+    _same(g.hypJacL2(10, G, n), ref, True)
