@@ -484,6 +484,75 @@ __device__ void inner64(double *const R, double *const Vl, const uint8_t *const 
   }
 }
 
+// Cholesky of 32 columns (the plain form's one-warp factor: a lane holds row
+// x, with TWO also row x + 32, in registers, the trailing entries moving one
+// register down a round; the next pivot's reciprocal root runs beside the
+// trailing updates).  A pivot that is not positive (a column dependent on the
+// previous ones to working accuracy) gives a zero column.  Rounds 32 - LIVE ..
+// 32 - LIVE + 7.  The factor of 64 columns took 43.4 K cycles with a barrier per
+// column and eight warps.
+// 1 / sqrt(d), the root and the reciprocal rounded one after the other
+__device__ __forceinline__ double pivot_inverse_ieee(const double d)
+{
+  const double piv = d > 0.0 ? __dsqrt_rn(d) : 0.0;
+  return piv > 0.0 ? __drcp_rn(piv) : 0.0;
+}
+
+__device__ __forceinline__ double pivot_inverse_try(const double d, bool &ok)
+{
+  bool ok_s, ok_r;
+  const double r = rcp_try(sqrt_try(d, ok_s), ok_r);
+  ok = ok_s && ok_r && rsqrt_range(d);
+  return r;
+}
+
+template <bool TWO, unsigned LIVE>
+__device__ __forceinline__ void chol_panel_rounds(double *const A, const unsigned x, double (&a)[32], double (&b)[32],
+                                                  double &rs, double &diag)
+{
+#pragma unroll 1
+  for (unsigned k = 32u - LIVE; k < 40u - LIVE; ++k) {
+    const double l = a[0] * rs, m = TWO ? b[0] * rs : 0.0;
+    if (x == k)
+      diag = a[0];
+    double *const col = A + k * kLd;
+    if (x > k)
+      col[x] = l;
+    if (TWO)
+      col[x + 32u] = m;
+    const double pv = __shfl_sync(0xffffffffu, __fma_rn(-l, l, a[1]), (k + 1u) & 31u);
+    bool ok;
+    rs = pivot_inverse_try(pv, ok);
+    __syncwarp();
+#pragma unroll
+    for (unsigned j = 1u; j < LIVE; ++j) { // past the last column: read and never used
+      const double f = col[k + j];
+      a[j - 1u] = __fma_rn(-l, f, a[j]);
+      if (TWO)
+        b[j - 1u] = __fma_rn(-m, f, b[j]);
+    }
+    if (!ok)
+      rs = pivot_inverse_ieee(pv);
+  }
+}
+
+template <bool TWO> __device__ __forceinline__ void chol_panel(double *const A, const unsigned x)
+{
+  double a[32], b[32], diag = 0.0;
+#pragma unroll
+  for (unsigned j = 0u; j < 32u; ++j) {
+    a[j] = A[j * kLd + x];
+    b[j] = TWO ? A[j * kLd + x + 32u] : 0.0;
+  }
+  double rs = pivot_inverse_ieee(__shfl_sync(0xffffffffu, a[0], 0));
+  __syncwarp();
+  chol_panel_rounds<TWO, 32u>(A, x, a, b, rs, diag);
+  chol_panel_rounds<TWO, 24u>(A, x, a, b, rs, diag);
+  chol_panel_rounds<TWO, 16u>(A, x, a, b, rs, diag);
+  chol_panel_rounds<TWO, 8u>(A, x, a, b, rs, diag);
+  A[x * kLd + x] = diag > 0.0 ? __dsqrt_rn(diag) : 0.0;
+}
+
 // the update's B operand diag(2^e_k) V_loc of one matrix: its digit planes
 // (K-major, n = output column j, k = pair column; the columns of each half
 // apart) and the exponents h_j, written to global memory.  Thread
@@ -719,78 +788,34 @@ __global__ void __launch_bounds__(kThreads, 1) sp_pair_kernel(const __grid_const
   if (rec)
     P.clk[1] = clock64() - t_start;
 
-  // Cholesky of the Gram matrix (lower triangle, in place), one barrier per
-  // column: in round k warp 0 updates column k + 1 by column k and pivots it
-  // (L(i, j) = A(i, j) / sqrt(A(j, j)), by the reciprocal), while warps 1..7
-  // update columns k + 2 .. 63 by column k.  A pivot that is not positive (a
-  // column dependent on the previous ones to working accuracy) gives a zero
-  // column of L.  Lane x holds rows x and x + 32.
+  // Cholesky of the Gram matrix (lower triangle, in place): the left 32 columns
+  // by warp 0, the rest of the matrix less their products by all, then the
+  // last 32 columns by warp 0
+  if (warp == 0u)
+    chol_panel<true>(R, lane);
+  __syncthreads();
   {
-    const auto pivot = [&](const unsigned j) {
-      __syncwarp();
-      const double d = R[j * kLd + j];
-      const double piv = d > 0.0 ? __dsqrt_rn(d) : 0.0, inv = piv > 0.0 ? __drcp_rn(piv) : 0.0;
-      __syncwarp();
+    const unsigned i = 32u + lane;
+    double acc[4];
 #pragma unroll
-      for (unsigned h = 0u; h < 2u; ++h) {
-        const unsigned i = lane + 32u * h;
-        if (i > j)
-          R[j * kLd + i] *= inv;
-        else if (i == j)
-          R[j * kLd + j] = piv;
-      }
-    };
-    if (warp == 0u)
-      pivot(0u);
-    __syncthreads();
-    for (unsigned k = 0u; k + 1u < 64u; ++k) {
-      if (warp == 0u) {
-        const unsigned j = k + 1u;
-        const double ljk = R[k * kLd + j];
+    for (unsigned u = 0u; u < 4u; ++u)
+      acc[u] = R[(32u + warp + 8u * u) * kLd + i];
+#pragma unroll 4
+    for (unsigned k = 0u; k < 32u; ++k) {
+      const double li = -R[k * kLd + i];
 #pragma unroll
-        for (unsigned h = 0u; h < 2u; ++h) {
-          const unsigned i = lane + 32u * h;
-          if (i >= j)
-            R[j * kLd + i] = __fma_rn(-R[k * kLd + i], ljk, R[j * kLd + i]);
-        }
-        pivot(j);
-      }
-      else {
-        // the columns of a round are independent: three at a time, so that
-        // their shared-memory loads overlap (each entry's operations unchanged)
-        const double l0 = R[k * kLd + lane], l1 = R[k * kLd + lane + 32u];
-        unsigned j = k + 1u + warp;
-#pragma unroll 1
-        for (; j + 14u < 64u; j += 21u) {
-          double ljk[3], a0[3], a1[3];
-#pragma unroll
-          for (unsigned u = 0u; u < 3u; ++u) {
-            const unsigned jj = j + 7u * u;
-            ljk[u] = R[k * kLd + jj];
-            a0[u] = R[jj * kLd + lane];
-            a1[u] = R[jj * kLd + lane + 32u];
-          }
-#pragma unroll
-          for (unsigned u = 0u; u < 3u; ++u) {
-            const unsigned jj = j + 7u * u;
-            if (lane >= jj)
-              R[jj * kLd + lane] = __fma_rn(-l0, ljk[u], a0[u]);
-            if (lane + 32u >= jj)
-              R[jj * kLd + lane + 32u] = __fma_rn(-l1, ljk[u], a1[u]);
-          }
-        }
-#pragma unroll 1
-        for (; j < 64u; j += 7u) {
-          const double ljk = R[k * kLd + j];
-          if (lane >= j)
-            R[j * kLd + lane] = __fma_rn(-l0, ljk, R[j * kLd + lane]);
-          if (lane + 32u >= j)
-            R[j * kLd + lane + 32u] = __fma_rn(-l1, ljk, R[j * kLd + lane + 32u]);
-        }
-      }
-      __syncthreads();
+      for (unsigned u = 0u; u < 4u; ++u)
+        acc[u] = __fma_rn(li, R[k * kLd + 32u + warp + 8u * u], acc[u]);
     }
+#pragma unroll
+    for (unsigned u = 0u; u < 4u; ++u)
+      if (i >= 32u + warp + 8u * u)
+        R[(32u + warp + 8u * u) * kLd + i] = acc[u];
   }
+  __syncthreads();
+  if (warp == 0u)
+    chol_panel<false>(R + 32u * kLd + 32u, lane);
+  __syncthreads();
   // R = L^T (upper), V_loc = I
   for (unsigned e = tid; e < 64u * 64u; e += kThreads) {
     const unsigned i = e & 63u, j = e >> 6; // R(i, j) = L(j, i) for i <= j: both from the lower triangle
