@@ -85,6 +85,8 @@ struct Params {
   uint32_t *cmaxG; // [2][ncol]: high word of the largest |entry| of each column, by step parity
   uint32_t *cmaxV; // [2][ncol]
   uint8_t *bop;    // per pair: the update's B operands (G, then V): kBopBytes each
+  double *vloc;    // per pair [64][64]: V_loc of this step, when V is updated beside the next step's
+                   // pair kernel (sp_bopv_kernel makes its B operand); null: the pair kernel does
   double *G, *V;
   unsigned ldG, ldV;
   unsigned nrow, ncol, nplus, pairs, step, parity, s0steps, nswp0;
@@ -617,7 +619,7 @@ __global__ void __launch_bounds__(kThreads, 1) sp_pair_kernel(const __grid_const
   if (tid < 64u) {
     const unsigned gc = (tid < kBW) ? iBlk * kBW + tid : jBlk * kBW + tid - kBW;
     eG[tid] = col_exp(P.cmaxG[P.parity * P.ncol + gc]);
-    eV[tid] = ACCV ? col_exp(P.cmaxV[P.parity * P.ncol + gc]) : 0;
+    eV[tid] = (ACCV && !P.vloc) ? col_exp(P.cmaxV[P.parity * P.ncol + gc]) : 0;
   }
   for (unsigned i = tid; i < P.s0steps * 64u; i += kThreads)
     s0[i] = P.strat0[i];
@@ -849,12 +851,17 @@ __global__ void __launch_bounds__(kThreads, 1) sp_pair_kernel(const __grid_const
   // the update's B operands, the counters, and the next step's column maxima cleared
   uint8_t *const bop = P.bop + (size_t)pair * (ACCV ? 2u : 1u) * kBopBytes;
   bop_write(Vl, eG, bop);
-  if (ACCV)
+  if (ACCV && P.vloc) {
+    double *const out = P.vloc + (size_t)pair * 4096u;
+    for (unsigned e = tid; e < 4096u; e += kThreads)
+      out[e] = Vl[(e >> 6) * kLd + (e & 63u)];
+  }
+  else if (ACCV)
     bop_write(Vl, eV, bop + kBopBytes);
   if (tid < 64u) {
     const unsigned gc = (tid < kBW) ? iBlk * kBW + tid : jBlk * kBW + tid - kBW;
     P.cmaxG[(P.parity ^ 1u) * P.ncol + gc] = 0u;
-    if (ACCV)
+    if (ACCV && !P.vloc)
       P.cmaxV[(P.parity ^ 1u) * P.ncol + gc] = 0u;
   }
   if (tid == 0u && blk_s) {
@@ -865,6 +872,27 @@ __global__ void __launch_bounds__(kThreads, 1) sp_pair_kernel(const __grid_const
   }
   if (rec)
     P.clk[4] = clock64() - t_start;
+}
+
+// The B operand of V's update from the V_loc that the pair kernel left (P.vloc),
+// with the column scales that V's previous update left; clears the maxima that
+// this step's will write.  One CTA per block pair.
+__global__ void __launch_bounds__(kThreads) sp_bopv_kernel(const __grid_constant__ Params P)
+{
+  __shared__ double Vl[64u * kLd];
+  __shared__ int eV[64];
+  const unsigned tid = threadIdx.x, pair = blockIdx.x;
+  const uint16_t *const blk = P.strat1 + ((size_t)P.step * P.pairs + pair) * 2u;
+  const double *const in = P.vloc + (size_t)pair * 4096u;
+  for (unsigned e = tid; e < 4096u; e += kThreads)
+    Vl[(e >> 6) * kLd + (e & 63u)] = in[e];
+  if (tid < 64u) {
+    const unsigned gc = (tid < kBW) ? blk[0] * kBW + tid : blk[1] * kBW + tid - kBW;
+    eV[tid] = col_exp(P.cmaxV[P.parity * P.ncol + gc]);
+    P.cmaxV[(P.parity ^ 1u) * P.ncol + gc] = 0u;
+  }
+  __syncthreads();
+  bop_write(Vl, eV, P.bop + ((size_t)pair * 2u + 1u) * kBopBytes);
 }
 
 // ---------------------------------------------------------------------------
@@ -1297,6 +1325,10 @@ struct SplitCtx {
   uint8_t *d_bop = nullptr;
   size_t bop_cap = 0u;
   unsigned long long *d_cnt = nullptr, *h_cnt = nullptr;
+  double *d_vloc = nullptr;    // two steps' V_loc (V updated beside the next pair kernel)
+  size_t vloc_cap = 0u;
+  cudaStream_t side = nullptr; // that update's stream
+  cudaEvent_t main_ev = nullptr, side_ev[2] = {nullptr, nullptr};
   long long *d_clk = nullptr;  // 16 words: phase clocks of the last pair launch, update phase sums
   std::vector<cudaEvent_t> ev; // profiling: two per outer step
 };
@@ -1366,13 +1398,32 @@ template <bool S, bool A> cudaError_t set_attrs()
   return cudaFuncSetAttribute(sp_update_kernel<A>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kUpdSmem);
 }
 
+// V's update of step p on the side stream, beside what the main stream does
+// after main_ev: its B operands, then the update on the SMs that the next
+// step's pair kernel leaves free; done: after the B operands (V_loc is read)
+cudaError_t launch_side(SplitCtx &c, Params p, const cudaEvent_t done)
+{
+  cudaError_t e = cudaStreamWaitEvent(c.side, c.main_ev, 0u);
+  if (e != cudaSuccess)
+    return e;
+  sp_bopv_kernel<<<p.pairs, kThreads, 0u, c.side>>>(p);
+  if ((e = cudaGetLastError()) != cudaSuccess || (e = cudaEventRecord(done, c.side)) != cudaSuccess)
+    return e;
+  p.tilesG = 0u;
+  const unsigned items = p.pairs * p.tilesV, ctas = p.sms - p.pairs;
+  sp_update_kernel<true><<<items < ctas ? items : ctas, kThreads, kUpdSmem, c.side>>>(p);
+  return cudaGetLastError();
+}
+
 template <bool S, bool A>
-cudaError_t launch_step(const Params &p, const cudaStream_t st, cudaEvent_t e0, cudaEvent_t e1)
+cudaError_t launch_step(Params p, const cudaStream_t st, cudaEvent_t e0, cudaEvent_t e1)
 {
   sp_pair_kernel<S, A><<<p.pairs, kThreads, kPairSmem, st>>>(p);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess)
     return e;
+  if (p.vloc)
+    p.tilesV = 0u; // V's tiles are the side stream's
   if (e0 && (e = cudaEventRecord(e0, st)) != cudaSuccess)
     return e;
   const unsigned items = p.pairs * (p.tilesG + p.tilesV);
@@ -1489,11 +1540,38 @@ int split_sweeps(const unsigned routine, const unsigned nrow, const unsigned nco
   }
   sp_colmax_kernel<<<(ncol + 7u) / 8u, 256u, 0u, st>>>(dG, nrow, ncol, lddG, p.cmaxG);
   SP_CUDA(cudaGetLastError(), "column maxima of G");
+  // V enters no later step's Gram matrix, so its update of a step can run
+  // beside the next step's pair kernel, one CTA per block pair, on the SMs that
+  // kernel leaves free: where those SMs do it in no more time than the pair
+  // kernel takes (tiles of 8 K cycles against 2.5 K cycles per 64 rows of the
+  // Gram products and 130 K of the rest), else it would delay the next update.
+  const bool prof = profiling();
+  const bool beside = full && !prof && p.pairs < p.sms &&
+                      (size_t)p.pairs * p.tilesV * 8000u <=
+                          (size_t)(p.sms - p.pairs) * ((nrow + 63u) / 64u * 2500u + 130000u);
+  if (beside) {
+    if (const int r = grow(c.d_vloc, c.vloc_cap, 2u * (size_t)pairs * 4096u, "cudaMalloc(V_loc)"))
+      return r;
+    if (!c.side) {
+      SP_CUDA(cudaStreamCreateWithFlags(&c.side, cudaStreamNonBlocking), "side stream");
+      SP_CUDA(cudaEventCreateWithFlags(&c.main_ev, cudaEventDisableTiming), "event");
+      SP_CUDA(cudaEventCreateWithFlags(&c.side_ev[0], cudaEventDisableTiming), "event");
+      SP_CUDA(cudaEventCreateWithFlags(&c.side_ev[1], cudaEventDisableTiming), "event");
+    }
+  }
+  // whatever way this function is left, the side stream's work is over
+  struct Side {
+    cudaStream_t s;
+    ~Side()
+    {
+      if (s)
+        (void)cudaStreamSynchronize(s);
+    }
+  } side_guard{beside ? c.side : nullptr};
   SP_CUDA(cudaMemsetAsync(c.d_cnt + 1, 0, sizeof(unsigned long long), st), "clear error word");
   SP_CUDA(cudaMemsetAsync(c.d_clk + 5, 0, 5u * sizeof(long long), st), "clear update clocks");
   *glb_s = 0ull;
   *glb_b = 0ull;
-  const bool prof = profiling();
   if (prof)
     while (c.ev.size() < 2u * c.steps1) {
       cudaEvent_t e = nullptr;
@@ -1507,9 +1585,18 @@ int split_sweeps(const unsigned routine, const unsigned nrow, const unsigned nco
     for (unsigned s = 0u; s < c.steps1; ++s, ++gstep) {
       p.step = s;
       p.parity = gstep & 1u;
+      if (beside) {
+        p.vloc = c.d_vloc + (size_t)p.parity * pairs * 4096u;
+        if (gstep >= 2u) // V_loc of step gstep - 2 has been read
+          SP_CUDA(cudaStreamWaitEvent(st, c.side_ev[p.parity], 0u), "side event");
+      }
       SP_CUDA(launch_split_step(cdsort, full, p, st, prof ? c.ev[2u * s] : nullptr,
                                 prof ? c.ev[2u * s + 1u] : nullptr),
               "split step");
+      if (beside) { // after this step's update of G, with the next pair kernel
+        SP_CUDA(cudaEventRecord(c.main_ev, st), "main event");
+        SP_CUDA(launch_side(c, p, c.side_ev[p.parity]), "split update of V");
+      }
     }
     ++swp;
     SP_CUDA(cudaMemcpyAsync(c.h_cnt, c.d_cnt, 2u * sizeof(unsigned long long), cudaMemcpyDeviceToHost, st),
@@ -1522,7 +1609,7 @@ int split_sweeps(const unsigned routine, const unsigned nrow, const unsigned nco
         SP_CUDA(cudaEventElapsedTime(&t, c.ev[2u * s], c.ev[2u * s + 1u]), "cudaEventElapsedTime");
         ms += t;
       }
-    profile_add(2ull * c.steps1, prof ? c.steps1 : 0u, ms);
+    profile_add((beside ? 4ull : 2ull) * c.steps1, prof ? c.steps1 : 0u, ms);
     if ((int)c.h_cnt[1]) {
       set_error("a split-form kernel timed out waiting for its copies or products");
       return GJX_ERR_DEVICE;
@@ -1535,7 +1622,16 @@ int split_sweeps(const unsigned routine, const unsigned nrow, const unsigned nco
   }
   *glbSwp = swp;
   SP_CUDA(launch_initD(dG, dD, nrow, ncol, nplus, lddG, st), "initD");
+  if (beside) { // the last steps' updates of V; their errors count too
+    SP_CUDA(cudaStreamSynchronize(c.side), "split updates of V");
+    SP_CUDA(cudaMemcpyAsync(c.h_cnt, c.d_cnt, 2u * sizeof(unsigned long long), cudaMemcpyDeviceToHost, st),
+            "read counters");
+  }
   SP_CUDA(cudaStreamSynchronize(st), "initD");
+  if (beside && (int)c.h_cnt[1]) {
+    set_error("a split-form kernel timed out waiting for its copies or products");
+    return GJX_ERR_DEVICE;
+  }
   return 0;
 }
 

@@ -1,9 +1,9 @@
 """The routes of a single decomposition's outer steps against the fused step
 kernel with one CTA per block pair, which the other tests hold against the
-oracle: clusters of 2, 4 and 8 CTAs per pair; the update as a launch of its
-own, its stages dealt out to all SMs, with 1 to 8 CTAs per pair before it, with
-more pairs than SMs, with partial stages and with pairs that do not change.
-The same bits."""
+oracle: clusters of 8 CTAs per pair; the update as a launch of its own, its
+stages dealt out to all SMs, with 1 to 8 CTAs per pair before it, with more
+pairs than SMs, with partial stages and with pairs that do not change; and the
+split form with V updated beside the next step's pair kernel.  The same bits."""
 
 import numpy as np
 import pytest
@@ -75,3 +75,26 @@ def test_update_launch_with_unchanged_pairs(built):
     ref = _fused(g, 10, G, n)
     g.lib().gjx_set_sweep_mode(-1)
     _same(g.hypJacL2(10, G, n), ref, True)
+
+
+@pytest.mark.parametrize("m,n,nplus,alg", [(64, 64, 64, 11), (1088, 320, 100, 11), (2112, 2048, 2048, 3), (512, 512, 512, 10)])
+def test_split_form_with_v_beside(m, n, nplus, alg, built):
+    """Timed (gjx_profile) launches keep V's update on the main stream."""
+    import torch
+
+    import gpujachx_b200 as g
+    G = synth.make("graded" if nplus < n else "gaussian", m, n, 8)
+    g.init_strats(None, "cycwor", 32, "cycwor", n // 16)
+    runs = []
+    for timed in (True, False):
+        dG = torch.tensor(np.ascontiguousarray(G.T), device="cuda")
+        dV = torch.zeros((n, n), dtype=torch.float64, device="cuda")
+        dD = torch.zeros(n, dtype=torch.float64, device="cuda")
+        g.profile(timed)
+        counts = g.hypJacL2_split(alg, dG, nplus, dV, dD)
+        g.profile(False)
+        runs.append((counts, dG.cpu().numpy(), dV.cpu().numpy(), dD.cpu().numpy()))
+    a, b = runs
+    assert a[0] == b[0]
+    for x, y in zip(a[1:], b[1:]):
+        assert np.array_equal(x.view(np.uint64), y.view(np.uint64))
