@@ -629,15 +629,27 @@ int run_batch(const unsigned routine, const unsigned nmat, const unsigned *const
   int dev = 0, sms = 148;
   GJX_CUDA(cudaGetDevice(&dev), "cudaGetDevice");
   GJX_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "SM count");
-  unsigned width = (g_pairs_per_cta == 1u || g_pairs_per_cta == gjx::kWidthHalf ||
-                    g_pairs_per_cta == gjx::kWidthHalf2) ? g_pairs_per_cta : 2u;
-  int mode = g_batch_mode;
+  // Untuned: one launch per sweep, and by the block pairs of a step of the whole
+  // batch -- up to two per SM one pair per CTA of 8 warps (an SM's whole
+  // arithmetic for a pair: the chain of a matrix's steps is what takes the
+  // time), then one pair per CTA of 4 warps, two CTAs per SM, and from 8 per SM
+  // two pairs per CTA of 4 warps (throughput).  Before: two pairs per CTA of 8
+  // warps, one launch per step.  ms, pairs: before / 1 / 3 / 4 --
+  // 104: 22.7 / 13.2 / 16.1 / 26.9; 270: 67.4 / 49.6 / 52.7 / 87.2; 498: 33.8 /
+  // 28.3 / 21.1 / 28.4; 1468: 221 / 224 / 162.3 / 161.8; 2886: 387 / 430 / 306 / 293.
+  unsigned width = (items.size() <= 2u * (unsigned)sms)   ? 1u
+                   : (items.size() <= 8u * (unsigned)sms) ? gjx::kWidthHalf
+                                                          : gjx::kWidthHalf2;
+  if (g_pairs_per_cta)
+    width = g_pairs_per_cta;
+  // (very large batches: one launch per step, 36402 pairs 3745 against 3795)
+  int mode = (g_batch_mode >= 0) ? g_batch_mode : (items.size() <= 64u * (unsigned)sms) ? 1 : 0;
   {
     const auto t = g_batch_tuned.find(batch_key(nmat, nrow, ncol, nplus));
     if (t != g_batch_tuned.end()) {
       if (!g_pairs_per_cta)
         width = t->second.first;
-      if (mode < 0)
+      if (g_batch_mode < 0)
         mode = t->second.second;
     }
   }

@@ -115,8 +115,8 @@ void gjx_set_split(unsigned n);
  * 4 (batched form only: two block pairs per CTA of 4 warps, two such CTAs
  * per SM; the two pairs' serial phases run concurrently on 2 warps each), or
  * 0 (default): automatic -- the batched autotuner's
- * choice, else 2 in the batched form (gjx_hypJacL2_batched), and in the
- * per-step launches of a single matrix with one CTA per block pair when a
+ * choice, else 1, 3 or 4 by the batch's block pairs per step
+ * (gjx_hypJacL2_batched), and in the per-step launches of a single matrix with one CTA per block pair when a
  * step has more block pairs than the GPU has SMs (one wave of CTAs instead of
  * two); else 1.  The results are the same bits for every value. */
 void gjx_set_pairs_per_cta(unsigned w);
@@ -145,7 +145,8 @@ int gjx_autotune(unsigned routine, unsigned nrow, unsigned ncol, unsigned nplus,
 void gjx_autotune_clear(void);
 
 /* The batched form's launches: -1 (default) the tuned choice
- * (gjx_autotune_batched), else one launch per outer step index; 0 one launch
+ * (gjx_autotune_batched), else one launch per sweep up to about ten thousand
+ * block pairs per step and one per outer step index above; 0 one launch
  * per outer step index for the whole batch (every active matrix advances one
  * step), replayed from a CUDA graph; 1 one launch per sweep of the whole
  * batch, in which a CTA takes (matrix, step, pair) items in step order and
