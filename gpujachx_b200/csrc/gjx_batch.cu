@@ -55,16 +55,14 @@ __global__ void __launch_bounds__(kThreads, 1) l1_batch_kernel(const __grid_cons
         pair_step<SORT, ACCV, 1u>(m.p, B.kstep[e >> 16u] % m.steps1, e & 0xffffu, 0u, sm);
         __syncthreads();
         if (threadIdx.x == 0u)
-          for (unsigned k = 0u; k < 8u; ++k)
-            mbar_inval(&bars[k]);
+          inval_bars(bars);
         __syncthreads();
       }
       continue;
     }
     __syncthreads();
     if (threadIdx.x == 0u)
-      for (unsigned k = 0u; k < 8u; ++k)
-        mbar_inval(&bars[k]);
+      inval_bars(bars);
     __syncthreads();
   }
 }

@@ -50,8 +50,7 @@ __global__ void __launch_bounds__(kThreads, 1) l1_batch_flow_kernel(const __grid
   auto inval = [&]() {
     __syncthreads();
     if (tid == 0u)
-      for (unsigned k = 0u; k < 8u; ++k)
-        mbar_inval(&bars[k]);
+      inval_bars(bars);
     __syncthreads();
   };
   for (;;) {

@@ -46,10 +46,11 @@ __global__ void __launch_bounds__(kNThreads, 2) l1_stepn_kernel(const __grid_con
 // for all block pairs (P.vt, P.vflag).  The 256-row stages of all pairs, in
 // order, are dealt out evenly to one CTA per SM; a CTA takes a contiguous run,
 // so its transform changes rarely (two buffers, the next pair's loaded with
-// its first stage).  Stages as in pair_step with three buffers.
+// its first stage).  Stages as in pair_step with three buffers, the warps not
+// waiting for one another.
 // ---------------------------------------------------------------------------
 constexpr unsigned kUOffVT = 3u * kUpdStage;
-constexpr unsigned kUOffBar = kUOffVT + 2u * kTransform; // [0..2] stages, [3..4] transforms
+constexpr unsigned kUOffBar = kUOffVT + 2u * kTransform; // [0..2] stages, [3..4] transforms, [5..7] stages done
 constexpr unsigned kUSmemDoubles = kUOffBar + 8u;
 static_assert(kUSmemDoubles * sizeof(double) <= 227u * 1024u, "three stages and two transforms must fit");
 
@@ -92,67 +93,92 @@ __global__ void __launch_bounds__(kThreads, 1) l1_update_kernel(const __grid_con
     bulk_g2s(sm + kUOffVT + (m & 1u) * kTransform, P.vt + (size_t)pair * kTransform, kTransform * 8u,
              &bars[3u + (m & 1u)]);
   };
+  const auto store = [&](const unsigned i, const unsigned n) { // one thread: stage i, the n-th, back
+    const CUtensorMap *tm;
+    int piece, ci, cj;
+    stage_at(i, tm, piece, ci, cj);
+    const double *const st = sm + (n % 3u) * kUpdStage;
+    tma_store_3d(tm, st, 0, piece, ci);
+    tma_store_3d(tm, st + 16u * kUpdColLd, 0, piece, cj);
+    bulk_commit();
+  };
+  const auto wait_done = [&](const unsigned n) { return mbar_wait_bounded(&bars[5u + n % 3u], (n / 3u) & 1u, kWaitLimit); };
   unsigned i = live(first);
   if (i >= end)
     return;
+  __shared__ unsigned s_stop;
+  volatile unsigned *const stop = &s_stop; // a wait gave up: all warps leave
   if (tid == 0u) {
-    for (unsigned b = 0u; b < 5u; ++b)
-      mbar_init(&bars[b], 1u);
+    for (unsigned b = 0u; b < 8u; ++b)
+      mbar_init(&bars[b], (b < 5u) ? 1u : kThreads / 32u);
     mbar_fence_init();
+    *stop = 0u;
     load_vt(i / nst, 0u);
     load(i, 0u);
   }
   __syncthreads();
   const unsigned sub = lane & 7u, cg8 = lane >> 3;
-  bool fresh = true; // the transform of this stage's pair has not been waited for
-  for (unsigned n = 0u, m = 0u; i < end; ++n) { // the n-th stage, with the m-th transform
+  unsigned n = 0u, m = 0u, last = i, stages = 1u, transforms = 1u; // (the last two: thread 0's loads)
+  int fail = 0;
+  for (bool fresh = true; i < end; ++n) { // the n-th stage, with the m-th transform
     const unsigned j = live(i + 1u);
     const bool turn = j < end && j / nst != i / nst;
-    if (tid == 0u && j < end) {
-      bulk_wait_read_but1(); // the store of the stage before the last has read its buffer out
-      load(j, n + 1u);
-      if (turn) // every warp is past the transform before the last
-        load_vt(j / nst, m + 1u);
-    }
-    bool ok = !fresh || mbar_wait_bounded(&bars[3u + (m & 1u)], (m >> 1) & 1u, kWaitLimit);
-    ok = ok && mbar_wait_bounded(&bars[n % 3u], (n / 3u) & 1u, kWaitLimit);
-    const int fail = !__all_sync(0xffffffffu, ok);
-    double *const st = sm + (n % 3u) * kUpdStage;
-    if (!fail) {
-      double acc[4][8];
-      update_stage(st, sm + kUOffVT + (m & 1u) * kTransform, warp, sub, cg8, acc);
-      __syncwarp();
-      update_put(st, acc, warp, sub, cg8);
-      fence_async_shared();
-    }
-    if (__syncthreads_or(fail)) { // uniform decision; drain (bounded), report
-      if (tid == 0u) {
-        (void)mbar_wait_bounded(&bars[n % 3u], (n / 3u) & 1u, kWaitLimit / 8);
-        if (fresh)
-          (void)mbar_wait_bounded(&bars[3u + (m & 1u)], (m >> 1) & 1u, kWaitLimit / 8);
-        if (j < end)
-          (void)mbar_wait_bounded(&bars[(n + 1u) % 3u], ((n + 1u) / 3u) & 1u, kWaitLimit / 8);
-        if (turn)
-          (void)mbar_wait_bounded(&bars[3u + ((m + 1u) & 1u)], ((m + 1u) >> 1) & 1u, kWaitLimit / 8);
-        bulk_wait_all();
-        atomicOr(P.err, kErrWaitTimeout);
-      }
-      return;
-    }
     if (tid == 0u) {
-      const CUtensorMap *tm;
-      int piece, ci, cj;
-      stage_at(i, tm, piece, ci, cj);
-      tma_store_3d(tm, st, 0, piece, ci);
-      tma_store_3d(tm, st + 16u * kUpdColLd, 0, piece, cj);
-      bulk_commit();
+      if (n > 0u) {
+        if (wait_done(n - 1u))
+          store(last, n - 1u);
+        else
+          fail = 1;
+      }
+      if (j < end && !fail) {
+        bulk_wait_read_but1(); // the store of the stage before the last has read its buffer out
+        load(j, n + 1u);
+        ++stages;
+        if (turn) { // every warp is past the transform before the last
+          load_vt(j / nst, m + 1u);
+          ++transforms;
+        }
+      }
     }
+    bool ok = !fail && !*stop;
+    ok = ok && (!fresh || mbar_wait_bounded(&bars[3u + (m & 1u)], (m >> 1) & 1u, kWaitLimit));
+    ok = ok && mbar_wait_bounded(&bars[n % 3u], (n / 3u) & 1u, kWaitLimit);
+    fail = !__all_sync(0xffffffffu, ok);
+    if (fail) {
+      *stop = 1u;
+      break;
+    }
+    double *const st = sm + (n % 3u) * kUpdStage;
+    double acc[4][8];
+    update_stage(st, sm + kUOffVT + (m & 1u) * kTransform, warp, sub, cg8, acc);
+    __syncwarp();
+    update_put(st, acc, warp, sub, cg8);
+    fence_async_shared();
+    __syncwarp();
+    if (lane == 0u)
+      mbar_arrive(&bars[5u + n % 3u]);
     fresh = turn;
     m += turn ? 1u : 0u;
+    last = i;
     i = j;
   }
-  if (tid == 0u)
+  if (tid == 0u && !fail) {
+    if (wait_done(n - 1u))
+      store(last, n - 1u);
+    else
+      fail = 1;
+  }
+  fail = __syncthreads_or(fail);
+  if (tid == 0u) {
+    if (fail) { // the copies in flight land (bounded); report
+      for (unsigned q = (stages > 2u) ? stages - 2u : 0u; q < stages; ++q)
+        (void)mbar_wait_bounded(&bars[q % 3u], (q / 3u) & 1u, kWaitLimit / 8);
+      for (unsigned q = (transforms > 2u) ? transforms - 2u : 0u; q < transforms; ++q)
+        (void)mbar_wait_bounded(&bars[3u + (q & 1u)], (q >> 1) & 1u, kWaitLimit / 8);
+      atomicOr(P.err, kErrWaitTimeout);
+    }
     bulk_wait_all();
+  }
 }
 
 // the reference's alternative builds (P.variant: 1 -DUSE_QR, 2 -DUSE_DRMAC):
@@ -221,8 +247,7 @@ __global__ void __launch_bounds__(kThreads, 1) l1_sweep_kernel(const __grid_cons
       __threadfence();
       atomicAdd(P.ver + iB, 1u);
       atomicAdd(P.ver + jB, 1u);
-      for (unsigned k = 0u; k < 8u; ++k)
-        mbar_inval(&bars[k]);
+      inval_bars(bars);
     }
     __syncthreads();
   }

@@ -90,8 +90,24 @@ constexpr unsigned kOffR = kRegion;        // R, 32x32 (later B^T, 32x34)
 constexpr unsigned kOffVl = kOffR + 32u * kVTLd;
 constexpr unsigned kOffS0 = kOffVl + 1024u; // strat0 copy, 1024 bytes
 constexpr unsigned kOffRed = kOffS0 + 128u; // 32 unsigned
-constexpr unsigned kOffBar = kOffRed + 16u; // 8 mbarriers
-constexpr unsigned kSmemDoubles = kOffBar + 8u;
+constexpr unsigned kOffBar = kOffRed + 16u; // mbarriers: [0..3] Gram stages, [4..6] update stages landed,
+                                            // [8..10] update stages done (one arrival per warp)
+constexpr unsigned kBars = 11u;
+constexpr unsigned kSmemDoubles = kOffBar + 12u;
+
+// every step form of 8 warps starts with all of them initialised
+__device__ __forceinline__ void init_bars(uint64_t *const bars)
+{
+  for (unsigned b = 0u; b < kBars; ++b)
+    mbar_init(&bars[b], (b < 8u) ? 1u : kThreads / 32u); // < 8: one arrival with the expected bytes
+  mbar_fence_init();
+}
+
+__device__ __forceinline__ void inval_bars(uint64_t *const bars)
+{
+  for (unsigned b = 0u; b < kBars; ++b)
+    mbar_inval(&bars[b]);
+}
 
 inline size_t l1_smem_bytes() { return (size_t)kSmemDoubles * sizeof(double); }
 
@@ -888,11 +904,8 @@ __device__ __forceinline__ void pair_step(const StepParams &P, const unsigned st
 
   for (unsigned i = tid; i < 256u; i += kThreads)
     reinterpret_cast<uint32_t *>(s0)[i] = reinterpret_cast<const uint32_t *>(P.strat0)[i];
-  if (tid == 0u) {
-    for (unsigned b = 0u; b < 8u; ++b)
-      mbar_init(&bars[b], 1u); // one arrival with the expected bytes, the TMA engine completes it
-    mbar_fence_init();
-  }
+  if (tid == 0u)
+    init_bars(bars);
   __syncthreads();
 
   int failed = 0;
@@ -1024,55 +1037,83 @@ __device__ __forceinline__ void pair_step(const StepParams &P, const unsigned st
     VT[s * kVTLd + c] = E32(Vl, s, c);
   }
 
-  __syncthreads(); // VT ready
-  // stage i: thread 0 issues the copy of stage i + 1 into its buffer once the
-  // store that last used that buffer has read it out (with 2 buffers the
-  // store of stage i - 1, issued just before; with 3 that of stage i - 2, a
-  // stage ago); the warps compute stage i and put the results in place;
-  // after the barrier thread 0 stores them with two tensor copies, which
-  // overlap the next stage's arithmetic
+  // The warps do not wait for one another: a warp waits for stage i to land,
+  // computes it, puts its results in place (of operands that only it read) and
+  // arrives on the stage's done barrier.  Thread 0, before its own stage i, waits
+  // for stage i - 1 to be done, stores it with two tensor copies, and issues the
+  // copy of stage i + 1 once the store that last used that buffer has read it
+  // out (with 3 buffers that of stage i - 2, with 2 that of i - 1, issued just
+  // before).  So one warp's stores and barrier latencies overlap the other's
+  // arithmetic on its sub-partition (with a CTA barrier per stage they coincided).
   const unsigned rg = warp, sub = lane & 7u, cg8 = lane >> 3;
+  auto store_upd = [&](const unsigned i) { // one thread: this CTA's i-th stage back
+    const unsigned k = rank + i * NSPLIT;
+    const bool isG = k < nG;
+    const CUtensorMap *const tm = isG ? &P.tmG : &P.tmV;
+    const int piece = (int)(((isG ? k : (k - nG)) * kUpdRows) >> 5);
+    double *const sb = ubuf(i % NBUF);
+    tma_store_3d(tm, sb, 0, piece, (int)(iBlk * kNColB));
+    tma_store_3d(tm, sb + 16u * kUpdColLd, 0, piece, (int)(jBlk * kNColB));
+    bulk_commit();
+  };
+  auto wait_done = [&](const unsigned i) {
+    return mbar_wait_bounded(&bars[8u + (i % NBUF)], (i / NBUF) & 1u, kWaitLimit);
+  };
+  volatile unsigned *const stop = red + 16u; // a wait gave up: all warps leave
+  if (tid == 0u)
+    *stop = 0u;
+  __syncthreads();
+  unsigned issued = (nmine > 0u) ? 1u : 0u; // thread 0: copies issued
+  int fail = 0;
   for (unsigned i = 0u; i < nmine; ++i) {
-    if (tid == 0u && i + 1u < nmine) {
-      if (NBUF == 3u)
-        bulk_wait_read_but1();
-      else
-        bulk_wait_read();
-      issue_upd(i + 1u);
+    if (tid == 0u) {
+      if (i > 0u) {
+        if (wait_done(i - 1u))
+          store_upd(i - 1u);
+        else
+          fail = 1;
+      }
+      if (i + 1u < nmine && !fail) {
+        if (NBUF == 3u)
+          bulk_wait_read_but1();
+        else
+          bulk_wait_read();
+        issue_upd(i + 1u);
+        issued = i + 2u;
+      }
     }
     // a warp computes only if all its lanes saw the stage land
-    const int fail = !__all_sync(0xffffffffu, mbar_wait_bounded(&bars[4u + (i % NBUF)], (i / NBUF) & 1u,
-                                                                kWaitLimit));
+    fail = !__all_sync(0xffffffffu, !fail && !*stop &&
+                                        mbar_wait_bounded(&bars[4u + (i % NBUF)], (i / NBUF) & 1u, kWaitLimit));
+    if (fail) {
+      *stop = 1u;
+      break;
+    }
     double *const sb = ubuf(i % NBUF);
-    if (!fail) {
-      double acc[4][8]; // the whole warp computes (rows past the end: not stored)
-      update_stage(sb, VT, rg, sub, cg8, acc);
-      __syncwarp();
-      update_put(sb, acc, rg, sub, cg8);
-      fence_async_shared();
-    }
-    if (__syncthreads_or(fail)) { // uniform decision; drain (bounded), report
-      if (tid == 0u) {
-        (void)mbar_wait_bounded(&bars[4u + (i % NBUF)], (i / NBUF) & 1u, kWaitLimit / 8);
-        if (i + 1u < nmine)
-          (void)mbar_wait_bounded(&bars[4u + ((i + 1u) % NBUF)], ((i + 1u) / NBUF) & 1u, kWaitLimit / 8);
-        bulk_wait_all();
-        atomicOr(P.err, kErrWaitTimeout);
-      }
-      return;
-    }
-    if (tid == 0u) {
-      const unsigned k = rank + i * NSPLIT;
-      const bool isG = k < nG;
-      const CUtensorMap *const tm = isG ? &P.tmG : &P.tmV;
-      const int piece = (int)(((isG ? k : (k - nG)) * kUpdRows) >> 5);
-      tma_store_3d(tm, sb, 0, piece, (int)(iBlk * kNColB));
-      tma_store_3d(tm, sb + 16u * kUpdColLd, 0, piece, (int)(jBlk * kNColB));
-      bulk_commit();
-    }
+    double acc[4][8]; // the whole warp computes (rows past the end: not stored)
+    update_stage(sb, VT, rg, sub, cg8, acc);
+    __syncwarp();
+    update_put(sb, acc, rg, sub, cg8);
+    fence_async_shared();
+    __syncwarp();
+    if (lane == 0u)
+      mbar_arrive(&bars[8u + (i % NBUF)]);
   }
-  if (tid == 0u)
+  if (tid == 0u && nmine > 0u && !fail) {
+    if (wait_done(nmine - 1u))
+      store_upd(nmine - 1u);
+    else
+      fail = 1;
+  }
+  fail = __syncthreads_or(fail);
+  if (tid == 0u) {
+    if (fail) { // the copies in flight land (bounded); report
+      for (unsigned q = (issued > 2u) ? issued - 2u : 0u; q < issued; ++q)
+        (void)mbar_wait_bounded(&bars[4u + (q % NBUF)], (q / NBUF) & 1u, kWaitLimit / 8);
+      atomicOr(P.err, kErrWaitTimeout);
+    }
     bulk_wait_all(); // the stores are complete before the block pair counts as done
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -1112,11 +1153,8 @@ __device__ __forceinline__ void pair_step2(const StepParams &PA, const unsigned 
 
   for (unsigned i = tid; i < 256u; i += kThreads)
     reinterpret_cast<uint32_t *>(s0)[i] = reinterpret_cast<const uint32_t *>(PA.strat0)[i];
-  if (tid == 0u) {
-    for (unsigned b = 0u; b < 8u; ++b)
-      mbar_init(&bars[b], 1u);
-    mbar_fence_init();
-  }
+  if (tid == 0u)
+    init_bars(bars);
   __syncthreads();
 
   // ------------------------------ 1. Grams --------------------------------

@@ -998,11 +998,6 @@ __device__ __forceinline__ bool wait_or_abort(uint64_t *bar, const uint32_t pari
   return true;
 }
 
-__device__ __forceinline__ void mbar_arrive(uint64_t *bar)
-{
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-
 // named barrier id of n threads that also ORs their predicates: the same
 // answer in every participating thread
 __device__ __forceinline__ bool bar_or(const unsigned id, const unsigned n, const bool pred)
