@@ -16,7 +16,7 @@
 //      clusters) to 8 chains (one CTA per pair) of neighbouring columns x and
 //      one or two columns y.  The shares are exchanged through distributed shared memory,
 //      then one cluster barrier.
-//   2. 32x32 Cholesky by one warp, the trailing matrix in registers
+//   2. 32x32 Cholesky by two warps, the trailing matrix in registers
 //      (share/device_code_common_Cholesky.hpp:58-158).
 //   3. Inner Jacobi sweep(s) on R: per inner step each warp sums the dot
 //      products of its two pairs by register butterflies in the reference's
@@ -291,69 +291,95 @@ template <unsigned NSPLIT> struct GramAcc {
 };
 
 // ---------------------------------------------------------------------------
-// Right-looking Cholesky of the lower triangle held in R, by one warp with
-// the trailing matrix in registers: lane x holds row x, a[j] = A(x, k + j) in
-// round k.  A round scales column k (x > k: times rsqrt_rn(A(k,k))), then
-// every trailing entry takes A(x,j) = fma(-A(x,k), A(j,k), A(x,j)) and moves
-// one register down, so that a round's indices are constants.  Every entry
-// receives the reference's operations in the reference's order
+// Right-looking Cholesky of the lower triangle held in R, by two warps with the
+// trailing matrix in registers: lane x holds row x, warp 0 its columns 0 .. 15,
+// warp 1 its columns 16 .. 31, a[j] = A(x, k + j) in round k.  A round scales
+// column k (x > k: times rsqrt_rn(A(k,k))), then every trailing entry takes
+// A(x,j) = fma(-A(x,k), A(j,k), A(x,j)) and moves one register down, so that a
+// round's indices are constants.  Warp 0 takes rounds 0 .. 15, warp 1 follows it
+// with its columns (a barrier of the two per round) and takes the rest.  Every
+// entry receives the reference's operations in the reference's order
 // (share/device_code_common_Cholesky.hpp:58-158); entries above the diagonal
 // are computed too and never used.
 // The round's serial chain is the pivot: lane k + 1 updates its own diagonal
 // entry (its factor is its own), one shuffle hands it to all lanes, and its
 // rsqrt_rn runs beside the trailing updates, whose factors A(j,k) come back
 // from shared memory (column k of R, where they belong anyway) by broadcast
-// loads.  The square roots of the diagonal are taken together at the end.
-// No barrier inside.  With a column look-ahead over 8 warps and a barrier per
-// column the pivot's chain was barrier, loads, update, shuffle, reciprocal root
-// and root; this form takes 2 to 5 us less of a step (256x256: 44.8 -> 42.4 us
-// per step, 4096x2048: 132 -> 129.6).
+// loads: 4 cycles each, which is why one warp for all 32 columns took 6.4 us.
+// The square roots of the diagonal are taken together at the end.  With a
+// column look-ahead over 8 warps and a barrier per column the pivot's chain was
+// barrier, loads, update, shuffle, reciprocal root and root: 9.8 us.
 // Afterwards R = L^T with zeros below the diagonal.
 // ---------------------------------------------------------------------------
-// rounds 32 - LIVE .. 32 - LIVE + 7, LIVE columns alive in the first of them
-template <unsigned LIVE>
-__device__ __forceinline__ void chol_rounds(double *const R, const unsigned x, double (&a)[32], double &rs,
-                                            double &diag)
+// rounds END - LIVE .. END - LIVE + 7 of the columns up to END - 1, LIVE of them
+// alive in the first; with FEED each round's column is handed to warp 1
+template <unsigned END, unsigned LIVE, bool FEED>
+__device__ __forceinline__ void chol_rounds(double *const R, const unsigned x, double (&a)[16], double &rs,
+                                            double &diag, const unsigned feed)
 {
 #pragma unroll 1
-  for (unsigned k = 32u - LIVE; k < 40u - LIVE; ++k) {
+  for (unsigned k = END - LIVE; k < END - LIVE + 8u; ++k) {
     const double l = a[0] * rs;
     if (x == k)
       diag = a[0];
     double *const col = R + k * 32u;
     if (x > k)
       col[x] = l;
-    // the next pivot (for k = 31 the values below are past the last column and unused)
+    // the next pivot (for k = END - 1 the values below are past the last column and unused)
     const double pv = __shfl_sync(0xffffffffu, __fma_rn(-l, l, a[1]), (k + 1u) & 31u);
     bool ok;
     rs = rsqrt_try(pv, ok);
-    __syncwarp();
+    if (FEED)
+      bar_sync(feed, 64u);
+    else
+      __syncwarp();
 #pragma unroll
     for (unsigned j = 1u; j < LIVE; ++j)
       a[j - 1u] = __fma_rn(-l, col[k + j], a[j]);
-    if (!(ok && rsqrt_range(pv)) && k + 1u < 32u)
+    if (!(ok && rsqrt_range(pv)) && k + 1u < END)
       rs = rsqrt_rn_full(pv);
   }
 }
 
-// by a group of NW warps (thread gt of the group, named barrier bar): the
-// group's warp 0 factors, all transpose
+// by a group of NW warps (thread gt of the group, named barriers bar and bar +
+// 8): the group's warps 0 and 1 factor, all transpose
 template <unsigned NW>
 __device__ __forceinline__ void chol32_grp(double *const R, const unsigned gt, const unsigned bar)
 {
-  if (gt < 32u) {
-    const unsigned x = gt;
-    double a[32], diag = 0.0;
+  if (gt < 64u) {
+    const unsigned x = gt & 31u;
+    double a[16], diag = 0.0, rs;
+    if (gt < 32u) {
 #pragma unroll
-    for (unsigned j = 0u; j < 32u; ++j)
-      a[j] = E32(R, x, j);
-    double rs = rsqrt_rn(__shfl_sync(0xffffffffu, a[0], 0));
-    __syncwarp();
-    chol_rounds<32u>(R, x, a, rs, diag);
-    chol_rounds<24u>(R, x, a, rs, diag);
-    chol_rounds<16u>(R, x, a, rs, diag);
-    chol_rounds<8u>(R, x, a, rs, diag);
-    E32(R, x, x) = __dsqrt_rn(diag);
+      for (unsigned j = 0u; j < 16u; ++j)
+        a[j] = E32(R, x, j);
+      rs = rsqrt_rn(__shfl_sync(0xffffffffu, a[0], 0));
+      __syncwarp();
+      chol_rounds<16u, 16u, true>(R, x, a, rs, diag, bar + 8u);
+      chol_rounds<16u, 8u, true>(R, x, a, rs, diag, bar + 8u);
+      if (x < 16u)
+        E32(R, x, x) = __dsqrt_rn(diag);
+    }
+    else {
+#pragma unroll
+      for (unsigned j = 0u; j < 16u; ++j)
+        a[j] = E32(R, x, 16u + j);
+#pragma unroll 1
+      for (unsigned k = 0u; k < 16u; ++k) {
+        bar_sync(bar + 8u, 64u);
+        const double *const col = R + k * 32u;
+        const double l = col[x];
+#pragma unroll
+        for (unsigned j = 0u; j < 16u; ++j)
+          a[j] = __fma_rn(-l, col[16u + j], a[j]);
+      }
+      rs = rsqrt_rn(__shfl_sync(0xffffffffu, a[0], 16));
+      __syncwarp();
+      chol_rounds<32u, 16u, false>(R, x, a, rs, diag, 0u);
+      chol_rounds<32u, 8u, false>(R, x, a, rs, diag, 0u);
+      if (x >= 16u)
+        E32(R, x, x) = __dsqrt_rn(diag);
+    }
   }
   bar_sync(bar, NW * 32u);
   constexpr unsigned NV = 1024u / (NW * 32u);
