@@ -18,12 +18,12 @@
 //      then one cluster barrier.
 //   2. 32x32 Cholesky by two warps, the trailing matrix in registers
 //      (share/device_code_common_Cholesky.hpp:58-158).
-//   3. Inner Jacobi sweep(s) on R: per inner step each warp sums the dot
-//      products of its two pairs by register butterflies in the reference's
-//      order, half-warps compute the two rotations (branch-free; trigonometric
-//      or hyperbolic, optional KISS sorting) and every lane applies both to its
-//      row of R and V_loc; one barrier per step (share/device_code_nosort.hpp,
-//      share/device_code_cdsort.hpp, share/device_code_cdsort_KISS.hpp).
+//   3. Inner Jacobi sweep(s) on R: per inner step 16 lanes take each of the 16
+//      column pairs, sum its dot products in the reference's order, evaluate
+//      its rotation (branch-free; trigonometric or hyperbolic, optional KISS
+//      sorting) and apply it to their two rows of R and V_loc; one barrier per
+//      step (share/device_code_nosort.hpp, share/device_code_cdsort.hpp,
+//      share/device_code_cdsort_KISS.hpp).
 //      Steps 2 and 3 are deterministic, so every CTA of the cluster computes
 //      them itself and holds the same V_loc bit for bit.
 //   4. [G_i G_j] <- [G_i G_j] V_loc (and V likewise): 256-row stages brought
@@ -398,136 +398,107 @@ __device__ __forceinline__ void chol32_grp(double *const R, const unsigned gt, c
 }
 
 // ---------------------------------------------------------------------------
-// Inner Jacobi sweep(s) on R (32x32) accumulating V_loc.  Per inner step (16
-// disjoint column pairs) warp w owns pairs w and w + 8, lane x = row x:
-//   the six dot products (Dp, Dq, Apq of both pairs) by register butterflies
-//   in the reference's order (share/device_code_common_Kepler.hpp:26-74:
-//   lane i adds lane i^16, ^8, ^4, ^2, ^1; IEEE addition commutes, so every
-//   lane ends with lane 0's bits); lanes 0-15 compute pair w's rotation
-//   (branch-free), lanes 16-31 pair w+8's; the halves trade them with one
-//   shuffle; each lane applies both to its row of R and V_loc from the values
-//   it loaded at the start of the step.  One barrier per step.
+// Inner Jacobi sweep(s) on R (32x32) accumulating V_loc, by a group of NW warps
+// (8, 4 or 2; lane x, warp w of the group, named barrier bar).  An inner step
+// has 16 disjoint column pairs; LP = 2 NW lanes take one: lane i of them holds
+// NR = 32 / LP rows, i + LP g, of both columns of R and V_loc.
+//   The three dot products (Dp, Dq, Apq) are summed in the reference's order
+//   (share/device_code_common_Kepler.hpp:26-74: row r adds row r^16, then ^8, ^4,
+//   ^2, ^1; IEEE addition commutes): the first log2 NR levels are between the
+//   lane's own rows, the others butterflies within the LP lanes.  Every lane
+//   evaluates its pair's rotation (branch-free, so the pairs of a warp do not
+//   diverge) and applies it to its rows.  One barrier per step.
 // Every operation is the reference's (share/device_code_nosort.hpp:4-222,
 // share/device_code_cdsort.hpp:25-167, share/device_code_cdsort_KISS.hpp).
+// What bounds a step (8 warps): the SM executes one shuffle of a warp per cycle,
+// 6 per level of the butterfly and warp, and the rotation is a chain of 540
+// cycles.  With a row of two pairs per lane (all 32 lanes summing both pairs by
+// a reduce-scatter, then trading the two rotations) a warp had 37 shuffles a
+// step, here 24 (18 and 12 with 4 and 2 warps, before 36 and 54 and rotations
+// passed through shared memory).
+// The rows of neighbouring pairs' lanes are taken in another order (g ^ the
+// pair's number), which leaves every sum and keeps their loads in different
+// banks.
 // ---------------------------------------------------------------------------
-// apply rotation r to row x of columns p, q of R (values Gp, Gq, already
-// loaded) and of V_loc (Vp, Vq); mode 0 leaves them, 2 swaps the columns
-__device__ __forceinline__ void inner_apply(double *const R, double *const Vl, const unsigned p, const unsigned q,
-                                            const Rot &r, const unsigned x, const double Gp, const double Gq,
-                                            const double Vp, const double Vq)
-{
-  if (r.mode == 0)
-    return;
-  if (r.mode == 2) {
-    E32(R, x, p) = Gq;
-    E32(R, x, q) = Gp;
-    E32(Vl, x, p) = Vq;
-    E32(Vl, x, q) = Vp;
-    return;
-  }
-  double np = __fma_rn(r.t_, Gq, Gp), nq = __fma_rn(r.t, Gp, Gq);
-  double vp = __fma_rn(r.t_, Vq, Vp), vq = __fma_rn(r.t, Vp, Vq);
-  if (r.scale) {
-    np = r.c * np;
-    nq = r.c * nq;
-    vp = r.c * vp;
-    vq = r.c * vq;
-  }
-  const unsigned dp = r.swap ? q : p, dq = r.swap ? p : q;
-  E32(R, x, dp) = np;
-  E32(R, x, dq) = nq;
-  E32(Vl, x, dp) = vp;
-  E32(Vl, x, dq) = vq;
-}
-
-// by a group of NW warps (8 or 4; lane x, warp w of the group, named barrier
-// bar): warp w takes the NC = 8 / NW couples of pairs (w + c NW, w + c NW + 8)
-// of each inner step, interleaved
 template <bool SORT, unsigned NW>
 __device__ __forceinline__ void inner_sweeps(double *const R, double *const Vl, const uint8_t *const s0,
                                              const unsigned s0steps, const unsigned nswp, const int definite,
                                              const unsigned npos, unsigned *const red, const unsigned x,
                                              const unsigned w, const unsigned bar, unsigned &blk_s, unsigned &blk_b)
 {
-  constexpr unsigned NC = 8u / NW;
+  constexpr unsigned LP = 2u * NW, NR = 32u / LP;
   blk_s = 0u;
   blk_b = 0u;
-  const bool hb = x >= 16u; // this half computes the couple's second pair (else its first)
+  const unsigned sub = x / LP, i = x % LP;   // the pair's number in the warp, the lane's in the pair
+  const unsigned pair = w * (32u / LP) + sub; // the pair of the step
+  unsigned row[NR];
+#pragma unroll
+  for (unsigned g = 0u; g < NR; ++g)
+    row[g] = i + LP * (g ^ (sub & (16u / LP - 1u)));
   for (unsigned swp = 0u; swp < nswp; ++swp) {
-    unsigned ws = 0u, wb = 0u; // lanes 0 and 16: their pairs' counts
+    unsigned ws = 0u, wb = 0u; // lane 0 of each pair: its counts
     for (unsigned step = 0u; step < s0steps; ++step) {
-      const uint8_t *const st = s0 + step * 32u;
-      unsigned pa[NC], qa[NC], pb[NC], qb[NC];
-      double Gpa[NC], Gqa[NC], Gpb[NC], Gqb[NC], Vpa[NC], Vqa[NC], Vpb[NC], Vqb[NC], v[NC][3];
+      const unsigned e = *reinterpret_cast<const uint16_t *>(s0 + step * 32u + 2u * pair), p = e & 255u, q = e >> 8;
+      double Gp[NR], Gq[NR], Vp[NR], Vq[NR], dp[NR], dq[NR], pq[NR];
 #pragma unroll
-      for (unsigned c = 0u; c < NC; ++c) {
-        const unsigned a = w + c * NW;
-        pa[c] = st[2u * a];
-        qa[c] = st[2u * a + 1u];
-        pb[c] = st[2u * a + 16u];
-        qb[c] = st[2u * a + 17u];
-        Gpa[c] = E32(R, x, pa[c]);
-        Gqa[c] = E32(R, x, qa[c]);
-        Gpb[c] = E32(R, x, pb[c]);
-        Gqb[c] = E32(R, x, qb[c]);
-        // V_loc of the same rows, loaded now so that the application waits for no load
-        Vpa[c] = E32(Vl, x, pa[c]);
-        Vqa[c] = E32(Vl, x, qa[c]);
-        Vpb[c] = E32(Vl, x, pb[c]);
-        Vqb[c] = E32(Vl, x, qb[c]);
-        // the butterfly as a reduce-scatter: at the first level (lane ^ 16)
-        // each lane keeps the products of its half's pair and receives the
-        // partner's products of the same pair; the other four levels stay
-        // within the half.  Every lane adds the same operands in the same
-        // order as the full butterfly would, with half the shuffles.
-        const double va[3] = {__fma_rn(Gpa[c], Gpa[c], 0.0), __fma_rn(Gqa[c], Gqa[c], 0.0),
-                              __fma_rn(Gpa[c], Gqa[c], 0.0)};
-        const double vb[3] = {__fma_rn(Gpb[c], Gpb[c], 0.0), __fma_rn(Gqb[c], Gqb[c], 0.0),
-                              __fma_rn(Gpb[c], Gqb[c], 0.0)};
+      for (unsigned g = 0u; g < NR; ++g) {
+        Gp[g] = E32(R, row[g], p);
+        Gq[g] = E32(R, row[g], q);
+      }
 #pragma unroll
-        for (unsigned i = 0u; i < 3u; ++i) {
-          const double other = __shfl_xor_sync(0xffffffffu, hb ? va[i] : vb[i], 16);
-          v[c][i] = (hb ? vb[i] : va[i]) + other;
+      for (unsigned g = 0u; g < NR; ++g) { // loaded now so that the application waits for no load
+        Vp[g] = E32(Vl, row[g], p);
+        Vq[g] = E32(Vl, row[g], q);
+      }
+#pragma unroll
+      for (unsigned g = 0u; g < NR; ++g) {
+        dp[g] = __fma_rn(Gp[g], Gp[g], 0.0);
+        dq[g] = __fma_rn(Gq[g], Gq[g], 0.0);
+        pq[g] = __fma_rn(Gp[g], Gq[g], 0.0);
+      }
+#pragma unroll
+      for (unsigned k = NR / 2u; k; k >>= 1u)
+#pragma unroll
+        for (unsigned g = 0u; g < k; ++g) {
+          dp[g] = dp[g] + dp[g + k];
+          dq[g] = dq[g] + dq[g + k];
+          pq[g] = pq[g] + pq[g + k];
         }
+#pragma unroll
+      for (unsigned k = LP / 2u; k; k >>= 1u) {
+        const double a = __shfl_xor_sync(0xffffffffu, dp[0], k), b = __shfl_xor_sync(0xffffffffu, dq[0], k),
+                     c = __shfl_xor_sync(0xffffffffu, pq[0], k);
+        dp[0] = dp[0] + a;
+        dq[0] = dq[0] + b;
+        pq[0] = pq[0] + c;
       }
-#pragma unroll
-      for (unsigned k = 8u; k; k >>= 1u) {
-        double o[NC][3];
-#pragma unroll
-        for (unsigned c = 0u; c < NC; ++c)
-#pragma unroll
-          for (unsigned i = 0u; i < 3u; ++i)
-            o[c][i] = __shfl_xor_sync(0xffffffffu, v[c][i], k);
-#pragma unroll
-        for (unsigned c = 0u; c < NC; ++c)
-#pragma unroll
-          for (unsigned i = 0u; i < 3u; ++i)
-            v[c][i] = v[c][i] + o[c][i];
+      unsigned a_s, a_b;
+      const Rot r = inner_rot<SORT>(dp[0], dq[0], pq[0], p, q, definite, npos, a_s, a_b);
+      if (i == 0u) {
+        ws += a_s;
+        wb += a_b;
       }
-      Rot r[NC];
+      // c = 1 multiplies exactly; a swap of the columns (mode 2) keeps the
+      // values; mode 0 leaves them
+      if (__any_sync(0xffffffffu, r.mode != 0)) {
+        const bool raw = SORT && r.mode == 2;
+        const unsigned to_p = (SORT && (raw || r.swap)) ? q : p, to_q = (SORT && (raw || r.swap)) ? p : q;
 #pragma unroll
-      for (unsigned c = 0u; c < NC; ++c) {
-        unsigned a_s, a_b;
-        r[c] = inner_rot<SORT>(v[c][0], v[c][1], v[c][2], hb ? pb[c] : pa[c], hb ? qb[c] : qa[c], definite, npos, a_s,
-                               a_b);
-        if (x == 0u || x == 16u) {
-          ws += a_s;
-          wb += a_b;
+        for (unsigned g = 0u; g < NR; ++g) {
+          const double np = r.c * __fma_rn(r.t_, Gq[g], Gp[g]), nq = r.c * __fma_rn(r.t, Gp[g], Gq[g]);
+          if (r.mode != 0) {
+            E32(R, row[g], to_p) = raw ? Gp[g] : np;
+            E32(R, row[g], to_q) = raw ? Gq[g] : nq;
+          }
         }
-      }
 #pragma unroll
-      for (unsigned c = 0u; c < NC; ++c) {
-        Rot o;
-        o.c = __shfl_xor_sync(0xffffffffu, r[c].c, 16);
-        o.t = __shfl_xor_sync(0xffffffffu, r[c].t, 16);
-        o.t_ = __shfl_xor_sync(0xffffffffu, r[c].t_, 16);
-        const int fl = __shfl_xor_sync(0xffffffffu, r[c].mode | (r[c].scale << 2) | (r[c].swap << 3), 16);
-        o.mode = fl & 3;
-        o.scale = (fl >> 2) & 1;
-        o.swap = (fl >> 3) & 1;
-        const Rot m = r[c]; // a value: selecting between two lvalues would take their addresses
-        inner_apply(R, Vl, pa[c], qa[c], hb ? o : m, x, Gpa[c], Gqa[c], Vpa[c], Vqa[c]);
-        inner_apply(R, Vl, pb[c], qb[c], hb ? m : o, x, Gpb[c], Gqb[c], Vpb[c], Vqb[c]);
+        for (unsigned g = 0u; g < NR; ++g) {
+          const double np = r.c * __fma_rn(r.t_, Vq[g], Vp[g]), nq = r.c * __fma_rn(r.t, Vp[g], Vq[g]);
+          if (r.mode != 0) {
+            E32(Vl, row[g], to_p) = raw ? Vp[g] : np;
+            E32(Vl, row[g], to_q) = raw ? Vq[g] : nq;
+          }
+        }
       }
       bar_sync(bar, NW * 32u);
     }
@@ -545,238 +516,6 @@ __device__ __forceinline__ void inner_sweeps(double *const R, double *const Vl, 
       tot_b += red[2u * k + 1u];
     }
     bar_sync(bar, NW * 32u);
-    if (tot_s) {
-      blk_s += tot_s;
-      blk_b += tot_b;
-    }
-    else
-      break;
-  }
-}
-
-// by a group of 4 warps (lane x, warp w of the group, named barrier bar):
-// warp w takes pairs w, w + 4, w + 8, w + 12 of each inner step, and quarter
-// k of the warp (lanes 8k .. 8k + 7) computes pair w + 4k's rotation.  The
-// twelve dot products go through a reduce-scatter: at level 16 each half
-// keeps its two pairs' products (lanes 0-15 pairs w, w + 4), at level 8 each
-// quarter its own pair's, levels 4, 2, 1 stay within the quarter -- the same
-// operands in the same order as the full butterfly, with one rotation to
-// evaluate per warp and step.  Every lane then applies the four rotations.
-// The four rotations of a warp reach its lanes through shared memory (rs: 16
-// doubles of this warp's own; the lane 8k writes pair k's, every lane reads
-// all four back with broadcast loads), not through shuffles.
-template <bool SORT>
-__device__ __forceinline__ void inner_sweeps_q(double *const R, double *const Vl, const uint8_t *const s0,
-                                               const unsigned s0steps, const unsigned nswp, const int definite,
-                                               const unsigned npos, unsigned *const red, const unsigned x,
-                                               const unsigned w, const unsigned bar, unsigned &blk_s,
-                                               unsigned &blk_b, double *const rs)
-{
-  blk_s = 0u;
-  blk_b = 0u;
-  const bool up = x >= 16u, odd = ((x >> 3) & 1u) != 0u;
-  const unsigned mine = w + 4u * (x >> 3); // the pair this lane's quarter evaluates
-  for (unsigned swp = 0u; swp < nswp; ++swp) {
-    unsigned ws = 0u, wb = 0u; // lanes 0, 8, 16, 24: their pairs' counts
-    for (unsigned step = 0u; step < s0steps; ++step) {
-      const uint8_t *const st = s0 + step * 32u;
-      unsigned p[4], q[4];
-      double Gp[4], Gq[4], Vp[4], Vq[4], v[4][3];
-#pragma unroll
-      for (unsigned k = 0u; k < 4u; ++k) {
-        p[k] = st[2u * (w + 4u * k)];
-        q[k] = st[2u * (w + 4u * k) + 1u];
-        Gp[k] = E32(R, x, p[k]);
-        Gq[k] = E32(R, x, q[k]);
-        Vp[k] = E32(Vl, x, p[k]);
-        Vq[k] = E32(Vl, x, q[k]);
-        v[k][0] = __fma_rn(Gp[k], Gp[k], 0.0);
-        v[k][1] = __fma_rn(Gq[k], Gq[k], 0.0);
-        v[k][2] = __fma_rn(Gp[k], Gq[k], 0.0);
-      }
-      const unsigned pm = st[2u * mine], qm = st[2u * mine + 1u];
-      double h[2][3], s[3];
-#pragma unroll
-      for (unsigned j = 0u; j < 2u; ++j)
-#pragma unroll
-        for (unsigned i = 0u; i < 3u; ++i) {
-          const double other = __shfl_xor_sync(0xffffffffu, up ? v[j][i] : v[2u + j][i], 16);
-          h[j][i] = (up ? v[2u + j][i] : v[j][i]) + other;
-        }
-#pragma unroll
-      for (unsigned i = 0u; i < 3u; ++i) {
-        const double other = __shfl_xor_sync(0xffffffffu, odd ? h[0][i] : h[1][i], 8);
-        s[i] = (odd ? h[1][i] : h[0][i]) + other;
-      }
-#pragma unroll
-      for (unsigned k = 4u; k; k >>= 1u) {
-        double o[3];
-#pragma unroll
-        for (unsigned i = 0u; i < 3u; ++i)
-          o[i] = __shfl_xor_sync(0xffffffffu, s[i], k);
-#pragma unroll
-        for (unsigned i = 0u; i < 3u; ++i)
-          s[i] = s[i] + o[i];
-      }
-      unsigned a_s, a_b;
-      const Rot r = inner_rot<SORT>(s[0], s[1], s[2], pm, qm, definite, npos, a_s, a_b);
-      if (!(x & 7u)) {
-        ws += a_s;
-        wb += a_b;
-        double *const e = rs + 4u * (x >> 3);
-        e[0] = r.c;
-        e[1] = r.t;
-        e[2] = r.t_;
-        e[3] = __longlong_as_double((long long)(r.mode | (r.scale << 2) | (r.swap << 3)));
-      }
-      __syncwarp();
-#pragma unroll
-      for (unsigned k = 0u; k < 4u; ++k) {
-        const double2 ct = *reinterpret_cast<const double2 *>(rs + 4u * k);
-        const double2 tf = *reinterpret_cast<const double2 *>(rs + 4u * k + 2u);
-        Rot o;
-        o.c = ct.x;
-        o.t = ct.y;
-        o.t_ = tf.x;
-        const int f = (int)__double_as_longlong(tf.y);
-        o.mode = f & 3;
-        o.scale = (f >> 2) & 1;
-        o.swap = (f >> 3) & 1;
-        inner_apply(R, Vl, p[k], q[k], o, x, Gp[k], Gq[k], Vp[k], Vq[k]);
-      }
-      bar_sync(bar, 128u);
-    }
-    ws = __reduce_add_sync(0xffffffffu, ws);
-    wb = __reduce_add_sync(0xffffffffu, wb);
-    if (x == 0u) {
-      red[2u * w] = ws;
-      red[2u * w + 1u] = wb;
-    }
-    bar_sync(bar, 128u);
-    unsigned tot_s = 0u, tot_b = 0u;
-#pragma unroll
-    for (unsigned k = 0u; k < 4u; ++k) {
-      tot_s += red[2u * k];
-      tot_b += red[2u * k + 1u];
-    }
-    bar_sync(bar, 128u);
-    if (tot_s) {
-      blk_s += tot_s;
-      blk_b += tot_b;
-    }
-    else
-      break;
-  }
-}
-
-// by a group of 2 warps (lane x, warp w of the group, named barrier bar):
-// warp w takes pairs w, w + 2, ..., w + 14 of each inner step, and eighth k
-// of the warp (lanes 4k .. 4k + 3) computes pair w + 2k's rotation.  The
-// reduce-scatter of inner_sweeps_q goes one level further: at level 16 each
-// half keeps four pairs' products, at 8 each quarter two, at 4 each eighth
-// its own, levels 2 and 1 stay within the eighth -- the same operands in the
-// same order as the full butterfly.  Every lane then applies the eight
-// rotations to its row.
-// The eight rotations of a warp reach its lanes through shared memory (rs:
-// 32 doubles of this warp's own; lane 4k writes pair k's), as in
-// inner_sweeps_q.
-template <bool SORT>
-__device__ __forceinline__ void inner_sweeps_e(double *const R, double *const Vl, const uint8_t *const s0,
-                                               const unsigned s0steps, const unsigned nswp, const int definite,
-                                               const unsigned npos, unsigned *const red, const unsigned x,
-                                               const unsigned w, const unsigned bar, unsigned &blk_s,
-                                               unsigned &blk_b, double *const rs)
-{
-  blk_s = 0u;
-  blk_b = 0u;
-  const bool up = x >= 16u, odd8 = ((x >> 3) & 1u) != 0u, odd4 = ((x >> 2) & 1u) != 0u;
-  const unsigned mine = w + 2u * (x >> 2); // the pair this lane's eighth evaluates
-  for (unsigned swp = 0u; swp < nswp; ++swp) {
-    unsigned ws = 0u, wb = 0u; // lanes 0, 4, ..., 28: their pairs' counts
-    for (unsigned step = 0u; step < s0steps; ++step) {
-      const uint8_t *const st = s0 + step * 32u;
-      unsigned p[8], q[8];
-      double Gp[8], Gq[8], Vp[8], Vq[8], v[8][3];
-#pragma unroll
-      for (unsigned k = 0u; k < 8u; ++k) {
-        p[k] = st[2u * (w + 2u * k)];
-        q[k] = st[2u * (w + 2u * k) + 1u];
-        Gp[k] = E32(R, x, p[k]);
-        Gq[k] = E32(R, x, q[k]);
-        Vp[k] = E32(Vl, x, p[k]);
-        Vq[k] = E32(Vl, x, q[k]);
-        v[k][0] = __fma_rn(Gp[k], Gp[k], 0.0);
-        v[k][1] = __fma_rn(Gq[k], Gq[k], 0.0);
-        v[k][2] = __fma_rn(Gp[k], Gq[k], 0.0);
-      }
-      const unsigned pm = st[2u * mine], qm = st[2u * mine + 1u];
-      double h4[4][3], h2[2][3], s[3];
-#pragma unroll
-      for (unsigned j = 0u; j < 4u; ++j)
-#pragma unroll
-        for (unsigned i = 0u; i < 3u; ++i) {
-          const double other = __shfl_xor_sync(0xffffffffu, up ? v[j][i] : v[4u + j][i], 16);
-          h4[j][i] = (up ? v[4u + j][i] : v[j][i]) + other;
-        }
-#pragma unroll
-      for (unsigned j = 0u; j < 2u; ++j)
-#pragma unroll
-        for (unsigned i = 0u; i < 3u; ++i) {
-          const double other = __shfl_xor_sync(0xffffffffu, odd8 ? h4[j][i] : h4[2u + j][i], 8);
-          h2[j][i] = (odd8 ? h4[2u + j][i] : h4[j][i]) + other;
-        }
-#pragma unroll
-      for (unsigned i = 0u; i < 3u; ++i) {
-        const double other = __shfl_xor_sync(0xffffffffu, odd4 ? h2[0][i] : h2[1][i], 4);
-        s[i] = (odd4 ? h2[1][i] : h2[0][i]) + other;
-      }
-#pragma unroll
-      for (unsigned k = 2u; k; k >>= 1u) {
-        double o[3];
-#pragma unroll
-        for (unsigned i = 0u; i < 3u; ++i)
-          o[i] = __shfl_xor_sync(0xffffffffu, s[i], k);
-#pragma unroll
-        for (unsigned i = 0u; i < 3u; ++i)
-          s[i] = s[i] + o[i];
-      }
-      unsigned a_s, a_b;
-      const Rot r = inner_rot<SORT>(s[0], s[1], s[2], pm, qm, definite, npos, a_s, a_b);
-      if (!(x & 3u)) {
-        ws += a_s;
-        wb += a_b;
-        double *const e = rs + 4u * (x >> 2);
-        e[0] = r.c;
-        e[1] = r.t;
-        e[2] = r.t_;
-        e[3] = __longlong_as_double((long long)(r.mode | (r.scale << 2) | (r.swap << 3)));
-      }
-      __syncwarp();
-#pragma unroll
-      for (unsigned k = 0u; k < 8u; ++k) {
-        const double2 ct = *reinterpret_cast<const double2 *>(rs + 4u * k);
-        const double2 tf = *reinterpret_cast<const double2 *>(rs + 4u * k + 2u);
-        Rot o;
-        o.c = ct.x;
-        o.t = ct.y;
-        o.t_ = tf.x;
-        const int f = (int)__double_as_longlong(tf.y);
-        o.mode = f & 3;
-        o.scale = (f >> 2) & 1;
-        o.swap = (f >> 3) & 1;
-        inner_apply(R, Vl, p[k], q[k], o, x, Gp[k], Gq[k], Vp[k], Vq[k]);
-      }
-      bar_sync(bar, 64u);
-    }
-    ws = __reduce_add_sync(0xffffffffu, ws);
-    wb = __reduce_add_sync(0xffffffffu, wb);
-    if (x == 0u) {
-      red[2u * w] = ws;
-      red[2u * w + 1u] = wb;
-    }
-    bar_sync(bar, 64u);
-    const unsigned tot_s = red[0] + red[2], tot_b = red[1] + red[3];
-    bar_sync(bar, 64u);
     if (tot_s) {
       blk_s += tot_s;
       blk_b += tot_b;
@@ -1156,8 +895,7 @@ __device__ __forceinline__ void pair_step(const StepParams &P, const unsigned st
 constexpr unsigned kOffR2 = kSmemDoubles; // pair B's R (later B^T), V_loc, counters
 constexpr unsigned kOffVl2 = kOffR2 + 32u * kVTLd;
 constexpr unsigned kOffRed2 = kOffVl2 + 1024u;
-constexpr unsigned kOffRot2 = kOffRed2 + 16u; // the rotations of the 8 warps (inner_sweeps_q), 16 doubles each
-constexpr unsigned kSmemDoubles2 = kOffRot2 + 128u;
+constexpr unsigned kSmemDoubles2 = kOffRed2 + 16u;
 
 inline size_t batch2_smem_bytes() { return (size_t)kSmemDoubles2 * sizeof(double); }
 
@@ -1306,8 +1044,7 @@ __device__ __forceinline__ void pair_step2(const StepParams &PA, const unsigned 
     unsigned npos;
     block_signature(P, grp ? iB : iA, grp ? jB : jA, definite, npos);
     unsigned blk_s, blk_b;
-    inner_sweeps_q<SORT>(R, Vl, s0, P.s0steps, P.nswp0, definite, npos, red, lane, gw, 1u + grp, blk_s, blk_b,
-                         sm + kOffRot2 + 16u * warp);
+    inner_sweeps<SORT, 4u>(R, Vl, s0, P.s0steps, P.nswp0, definite, npos, red, lane, gw, 1u + grp, blk_s, blk_b);
     if (gt == 0u) {
       add_counts(P, blk_s, blk_b);
       flags[grp] = (SORT || blk_s) ? 1u : 0u;
@@ -1390,7 +1127,7 @@ __device__ __forceinline__ unsigned ld_acquire(const unsigned *p)
 // One block pair on a CTA of 4 warps (batched form, two such CTAs per SM).
 // The arithmetic is that of pair_step with one CTA per pair -- the Gram
 // chains of pair_step with one CTA per pair on warps 0-2 (warp 3 issues the tile copies), the
-// Cholesky factorisation and quarter-warp inner sweeps of pair_step2's warp
+// Cholesky factorisation and inner sweeps of pair_step2's warp
 // groups, pair_step's update tiles (warp w takes row groups w and w + 4 of
 // every stage) -- so every matrix gets the bits of its single call.  Shared
 // memory (86 KB): the Gram's 4 stages of one 64-row tile, later one update
@@ -1408,8 +1145,7 @@ constexpr unsigned kNOffVl = kNOffR + 32u * kVTLd;
 constexpr unsigned kNOffS0 = kNOffVl + 1024u;
 constexpr unsigned kNOffRed = kNOffS0 + 128u;
 constexpr unsigned kNOffBar = kNOffRed + 16u; // [0..3] Gram stages, [4] the update buffer
-constexpr unsigned kNOffRot = kNOffBar + 8u; // the rotations of the 4 warps (inner_sweeps_q), 16 doubles each
-constexpr unsigned kNSmemDoubles = kNOffRot + 64u;
+constexpr unsigned kNSmemDoubles = kNOffBar + 8u;
 static_assert(2u * (kNSmemDoubles * sizeof(double) + 1024u) <= 228u * 1024u, "two CTAs per SM");
 inline size_t batchn_smem_bytes() { return (size_t)kNSmemDoubles * sizeof(double); }
 
@@ -1503,8 +1239,7 @@ __device__ __forceinline__ void pair_step_n(const StepParams &P, const unsigned 
   unsigned npos;
   block_signature(P, iBlk, jBlk, definite, npos);
   unsigned blk_s, blk_b;
-  inner_sweeps_q<SORT>(R, Vl, s0, P.s0steps, P.nswp0, definite, npos, red, lane, warp, 0u, blk_s, blk_b,
-                       sm + kNOffRot + 16u * warp);
+  inner_sweeps<SORT, 4u>(R, Vl, s0, P.s0steps, P.nswp0, definite, npos, red, lane, warp, 0u, blk_s, blk_b);
   if (tid == 0u)
     add_counts(P, blk_s, blk_b);
   if (apart) {
@@ -1568,8 +1303,8 @@ __device__ __forceinline__ void pair_step_n(const StepParams &P, const unsigned 
 // takes row groups w and w + 4 of every stage) run on the 4 warps, A's then
 // B's, as one stream of tiles and one of stages; their Cholesky
 // factorisations and inner sweeps run concurrently, warps 0-1 on A (named
-// barrier 1), warps 2-3 on B (barrier 2), with the eighth-warp reduce-scatter
-// of inner_sweeps_e.  Every entry gets the operations of pair_step in the
+// barrier 1), warps 2-3 on B (barrier 2).
+// Every entry gets the operations of pair_step in the
 // same order, so each matrix gets the bits of its single call.  Shared
 // memory (104 KB): the Gram's 4 stages of one tile, later one update buffer;
 // A's and B's R, V_loc and counters.
@@ -1581,8 +1316,7 @@ constexpr unsigned kN2OffVlB = kN2OffRB + 32u * kVTLd;
 constexpr unsigned kN2OffS0 = kN2OffVlB + 1024u;
 constexpr unsigned kN2OffRed = kN2OffS0 + 128u; // [0..3] A's counts, [4..7] B's, [8..9] flags
 constexpr unsigned kN2OffBar = kN2OffRed + 8u;  // [0..3] Gram stages, [4] the update buffer
-constexpr unsigned kN2OffRot = kN2OffBar + 8u; // the rotations of the 4 warps (inner_sweeps_e), 32 doubles each
-constexpr unsigned kN2SmemDoubles = kN2OffRot + 128u;
+constexpr unsigned kN2SmemDoubles = kN2OffBar + 8u;
 static_assert(2u * (kN2SmemDoubles * sizeof(double) + 1024u) <= 228u * 1024u, "two CTAs per SM");
 inline size_t batchn2_smem_bytes() { return (size_t)kN2SmemDoubles * sizeof(double); }
 
@@ -1700,8 +1434,8 @@ __device__ __forceinline__ void pair_step2n(const StepParams &PA, const unsigned
     unsigned npos;
     block_signature(P, grp ? iB : iA, grp ? jB : jA, definite, npos);
     unsigned blk_s, blk_b;
-    inner_sweeps_e<SORT>(R, Vl, s0, P.s0steps, P.nswp0, definite, npos, red + 4u * grp, lane, gw, 1u + grp, blk_s,
-                         blk_b, sm + kN2OffRot + 32u * warp);
+    inner_sweeps<SORT, 2u>(R, Vl, s0, P.s0steps, P.nswp0, definite, npos, red + 4u * grp, lane, gw, 1u + grp, blk_s,
+                           blk_b);
     if (gt == 0u) {
       add_counts(P, blk_s, blk_b);
       red[8u + grp] = (SORT || blk_s) ? 1u : 0u;
