@@ -91,15 +91,17 @@ constexpr unsigned kOffVl = kOffR + 32u * kVTLd;
 constexpr unsigned kOffS0 = kOffVl + 1024u; // strat0 copy, 1024 bytes
 constexpr unsigned kOffRed = kOffS0 + 128u; // 32 unsigned
 constexpr unsigned kOffBar = kOffRed + 16u; // mbarriers: [0..3] Gram stages, [4..6] update stages landed,
-                                            // [8..10] update stages done (one arrival per warp)
-constexpr unsigned kBars = 11u;
-constexpr unsigned kSmemDoubles = kOffBar + 12u;
+                                            // [8..10] update stages done (one arrival per warp),
+                                            // [11..14] Gram stages read (one arrival per Gram warp)
+constexpr unsigned kBars = 15u;
+constexpr unsigned kGramWarps = 3u; // warps 0-2 compute Gram entries
+constexpr unsigned kSmemDoubles = kOffBar + 16u;
 
 // every step form of 8 warps starts with all of them initialised
 __device__ __forceinline__ void init_bars(uint64_t *const bars)
 {
   for (unsigned b = 0u; b < kBars; ++b)
-    mbar_init(&bars[b], (b < 8u) ? 1u : kThreads / 32u); // < 8: one arrival with the expected bytes
+    mbar_init(&bars[b], (b < 8u) ? 1u : (b < 11u) ? kThreads / 32u : kGramWarps); // < 8: the expected bytes
   mbar_fence_init();
 }
 
@@ -205,7 +207,7 @@ template <unsigned NSPLIT> struct GramShape {
   static constexpr unsigned XU = (NSPLIT == 1u) ? 4u : (NSPLIT == 2u) ? 2u : 1u;
   static constexpr unsigned YU = (NSPLIT <= 4u) ? 2u : 1u;
   static constexpr unsigned LX = (NSPLIT == 1u) ? 1u : 2u;
-  static constexpr unsigned warps = 3u;
+  static constexpr unsigned warps = kGramWarps;
 };
 
 struct GramLane {
@@ -700,30 +702,41 @@ __device__ __forceinline__ void pair_step(const StepParams &P, const unsigned st
     }
   };
 
-  if (tid == kIssuer)
-    for (unsigned k = 0u; k + 1u < kGramStages && k < ngst; ++k)
+  // The Gram warps do not wait for one another: each waits for a stage to land,
+  // adds its tiles and arrives on the stage's read barrier; the issuer refills a
+  // stage when all have.  (With a CTA barrier per stage of two tiles the phase
+  // took 570 cycles a stage more than the tiles do.)
+  if (tid == kIssuer) {
+    for (unsigned k = 0u; k < ngst; ++k) {
+      if (k >= kGramStages &&
+          !mbar_wait_bounded(&bars[11u + k % kGramStages], (k / kGramStages - 1u) & 1u, kWaitLimit)) {
+        failed = 1;
+        break;
+      }
       issue_gram(k);
-  unsigned k = 0u;
-  for (; k < ngst; ++k) {
-    if (tid == kIssuer && k + kGramStages - 1u < ngst)
-      issue_gram(k + kGramStages - 1u); // into the buffer released at the end of stage k - 1
-    int fail = 0;
-    if (warp < GramShape<NSPLIT>::warps) {
-      if (!mbar_wait_bounded(&bars[k % kGramStages], (k / kGramStages) & 1u, kWaitLimit))
-        fail = 1;
-      else if (gl.on) {
+    }
+  }
+  else if (warp < kGramWarps) {
+    for (unsigned k = 0u; k < ngst; ++k) {
+      if (!__all_sync(0xffffffffu, mbar_wait_bounded(&bars[k % kGramStages], (k / kGramStages) & 1u, kWaitLimit))) {
+        failed = 1;
+        break;
+      }
+      if (gl.on) {
         const unsigned nt = min(kGramTiles, ntile - k * kGramTiles);
         for (unsigned t = 0u; t < nt; ++t)
           gacc.tile(stg + (k % kGramStages) * kGramStage + t * kGramTileLd, gl);
       }
+      __syncwarp();
+      if (lane == 0u)
+        mbar_arrive(&bars[11u + k % kGramStages]);
     }
-    failed = __syncthreads_or(fail); // uniform decision
-    if (failed)
-      break;
   }
+  failed = __syncthreads_or(failed); // uniform decision
   if (failed && tid == 0u) { // let the copies in flight land (bounded) before anything else, report
-    for (unsigned q = k; q < ngst && q < k + kGramStages; ++q)
-      (void)mbar_wait_bounded(&bars[q % kGramStages], (q / kGramStages) & 1u, kWaitLimit / 8);
+    for (unsigned s = 0u; s < kGramStages; ++s)
+      for (unsigned par = 0u; par < 2u; ++par)
+        (void)mbar_wait_bounded(&bars[s], par, kWaitLimit / 8);
     atomicOr(P.err, kErrWaitTimeout);
   }
   // our share of the lower triangle, into our R and the other CTAs' R
