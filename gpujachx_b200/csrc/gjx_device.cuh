@@ -380,6 +380,12 @@ __device__ __forceinline__ void bar_sync(const unsigned id, const unsigned nthre
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
 }
 
+// programmatic dependent launch: let the next launch of the stream be placed
+// (it waits in pdl_wait until this grid is complete and its writes visible);
+// both do nothing in a launch without the attribute
+__device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // ---------------------------------------------------------------------------
 // mbarrier + bulk-copy (TMA engine) helpers, with bounded waits
 // ---------------------------------------------------------------------------

@@ -13,6 +13,7 @@ template <bool SORT, bool ACCV, unsigned NSPLIT>
 __global__ void __launch_bounds__(kThreads, 1) l1_step_kernel(const __grid_constant__ StepParams P)
 {
   extern __shared__ __align__(128) double sm[];
+  pdl_launch();
   const unsigned rank = (NSPLIT > 1u) ? (blockIdx.x % NSPLIT) : 0u;
   pair_step<SORT, ACCV, NSPLIT, UpdBuffers<NSPLIT>::value>(P, P.step, blockIdx.x / NSPLIT, rank, sm);
 }
@@ -25,6 +26,7 @@ template <bool SORT, bool ACCV>
 __global__ void __launch_bounds__(kThreads, 1) l1_step2_kernel(const __grid_constant__ StepParams P)
 {
   extern __shared__ __align__(128) double sm[];
+  pdl_launch();
   const unsigned a = 2u * blockIdx.x;
   if (a + 1u < P.pairs)
     pair_step2<SORT, ACCV>(P, P.step, a, P, P.step, a + 1u, sm);
@@ -38,6 +40,7 @@ template <bool SORT>
 __global__ void __launch_bounds__(kNThreads, 2) l1_stepn_kernel(const __grid_constant__ StepParams P)
 {
   extern __shared__ __align__(128) double sm[];
+  pdl_launch();
   pair_step_n<SORT, false>(P, P.step, blockIdx.x, sm);
 }
 
@@ -103,6 +106,8 @@ __global__ void __launch_bounds__(kThreads, 1) l1_update_kernel(const __grid_con
     bulk_commit();
   };
   const auto wait_done = [&](const unsigned n) { return mbar_wait_bounded(&bars[5u + n % 3u], (n / 3u) & 1u, kWaitLimit); };
+  pdl_launch();
+  pdl_wait(); // the transforms, G and V are the launch before's
   unsigned i = live(first);
   if (i >= end)
     return;
@@ -435,13 +440,15 @@ template <bool S, bool A, unsigned N> static cudaError_t launch(const StepParams
   cfg.blockDim = dim3(kThreads);
   cfg.dynamicSmemBytes = step_smem_bytes(N);
   cfg.stream = s;
-  cudaLaunchAttribute at[1];
+  cudaLaunchAttribute at[2];
   at[0].id = cudaLaunchAttributeClusterDimension;
   at[0].val.clusterDim.x = N;
   at[0].val.clusterDim.y = 1;
   at[0].val.clusterDim.z = 1;
+  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = 2;
   return cudaLaunchKernelEx(&cfg, l1_step_kernel<S, A, N>, p);
 }
 
@@ -572,10 +579,27 @@ unsigned l1_split(const unsigned pairs, const unsigned nrow)
   return (pairs <= f.c4) ? 4u : (pairs <= f.c2) ? 2u : 1u;
 }
 
+// a launch that may be placed before the one before it in the stream is complete
+template <typename K>
+static cudaError_t launch_pdl(K *const kernel, const unsigned ctas, const unsigned threads, const size_t smem,
+                              const StepParams &p, cudaStream_t s)
+{
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(ctas);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, p);
+}
+
 template <bool S, bool A> static cudaError_t launch2(const StepParams &p, cudaStream_t s)
 {
-  l1_step2_kernel<S, A><<<(p.pairs + 1u) / 2u, kThreads, batch2_smem_bytes(), s>>>(p);
-  return cudaGetLastError();
+  return launch_pdl(l1_step2_kernel<S, A>, (p.pairs + 1u) / 2u, kThreads, batch2_smem_bytes(), p, s);
 }
 
 template <bool S, bool A, unsigned F> static cudaError_t launch_var(const StepParams &p, cudaStream_t s)
@@ -589,11 +613,8 @@ template <bool S, bool A, unsigned F> static cudaError_t launch_var(const StepPa
 static cudaError_t launch_factor(const bool sort, const StepParams &p, cudaStream_t s)
 {
   if (p.width == kWidthHalf) {
-    if (sort)
-      l1_stepn_kernel<true><<<p.pairs, kNThreads, batchn_smem_bytes(), s>>>(p);
-    else
-      l1_stepn_kernel<false><<<p.pairs, kNThreads, batchn_smem_bytes(), s>>>(p);
-    return cudaGetLastError();
+    return launch_pdl(sort ? l1_stepn_kernel<true> : l1_stepn_kernel<false>, p.pairs, kNThreads, batchn_smem_bytes(), p,
+                      s);
   }
   switch (p.split) {
   case 8u:
@@ -611,8 +632,7 @@ template <bool A> static cudaError_t launch_update(const StepParams &p, cudaStre
 {
   const unsigned nst = (p.nrow + kUpdRows - 1u) / kUpdRows + (A ? (p.ncol + kUpdRows - 1u) / kUpdRows : 0u);
   const unsigned total = p.pairs * nst;
-  l1_update_kernel<A><<<total < p.sms ? total : p.sms, kThreads, kUSmemDoubles * sizeof(double), s>>>(p);
-  return cudaGetLastError();
+  return launch_pdl(l1_update_kernel<A>, total < p.sms ? total : p.sms, kThreads, kUSmemDoubles * sizeof(double), p, s);
 }
 
 cudaError_t launch_l1_step(const bool sort, const bool accv, const StepParams &p, cudaStream_t s)

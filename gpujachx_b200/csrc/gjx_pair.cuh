@@ -674,6 +674,7 @@ __device__ __forceinline__ void pair_step(const StepParams &P, const unsigned st
   if (tid == 0u)
     init_bars(bars);
   __syncthreads();
+  pdl_wait(); // G, V and the counters are the launch before's
 
   int failed = 0;
   if constexpr (FAC != 0u) {
@@ -934,6 +935,8 @@ __device__ __forceinline__ void pair_step2(const StepParams &PA, const unsigned 
     init_bars(bars);
   __syncthreads();
 
+  pdl_wait();
+
   // ------------------------------ 1. Grams --------------------------------
   // stages 0 .. ngA-1 are A's, ngA .. ngA+ngB-1 B's
   const unsigned ntA = PA.nrow >> 6, ntB = PB.nrow >> 6;
@@ -1184,6 +1187,8 @@ __device__ __forceinline__ void pair_step_n(const StepParams &P, const unsigned 
     mbar_fence_init();
   }
   __syncthreads();
+
+  pdl_wait(); // G, V and the counters are the launch before's
 
   // ------------------------------ 1. Gram --------------------------------
   const unsigned ntile = P.nrow >> 6;
