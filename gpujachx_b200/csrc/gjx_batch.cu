@@ -93,8 +93,7 @@ __global__ void __launch_bounds__(kNThreads, 2) l1_batchn_kernel(const __grid_co
     pair_step_n<SORT, ACCV>(m.p, B.kstep[b] % m.steps1, e & 0xffffu, sm);
     __syncthreads();
     if (threadIdx.x == 0u)
-      for (unsigned k = 0u; k < 5u; ++k)
-        mbar_inval(&bars[k]);
+      inval_bars_n(bars);
     __syncthreads();
   }
 }
@@ -111,8 +110,7 @@ __global__ void __launch_bounds__(kNThreads, 2) l1_batchn2_kernel(const __grid_c
   auto inval = [&](uint64_t *const bars) {
     __syncthreads();
     if (threadIdx.x == 0u)
-      for (unsigned k = 0u; k < 5u; ++k)
-        mbar_inval(&bars[k]);
+      inval_bars_n(bars);
     __syncthreads();
   };
   for (;;) {

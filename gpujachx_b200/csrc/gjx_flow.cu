@@ -169,8 +169,7 @@ __global__ void __launch_bounds__(kNThreads, 2) l1_batchn_flow_kernel(const __gr
       __threadfence();
       atomicAdd(v + iB, 1u);
       atomicAdd(v + jB, 1u);
-      for (unsigned k = 0u; k < 5u; ++k)
-        mbar_inval(&bars[k]);
+      inval_bars_n(bars);
     }
     __syncthreads();
   }
@@ -220,8 +219,7 @@ __global__ void __launch_bounds__(kNThreads, 2) l1_batchn2_flow_kernel(const __g
   auto inval = [&](uint64_t *const bars) {
     __syncthreads();
     if (tid == 0u)
-      for (unsigned k = 0u; k < 5u; ++k)
-        mbar_inval(&bars[k]);
+      inval_bars_n(bars);
     __syncthreads();
   };
   for (;;) {

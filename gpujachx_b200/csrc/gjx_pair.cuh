@@ -1160,10 +1160,60 @@ constexpr unsigned kNOffR = kNRegion; // R, 32x32 (later B^T, 32x34)
 constexpr unsigned kNOffVl = kNOffR + 32u * kVTLd;
 constexpr unsigned kNOffS0 = kNOffVl + 1024u;
 constexpr unsigned kNOffRed = kNOffS0 + 128u;
-constexpr unsigned kNOffBar = kNOffRed + 16u; // [0..3] Gram stages, [4] the update buffer
-constexpr unsigned kNSmemDoubles = kNOffBar + 8u;
+constexpr unsigned kNOffBar = kNOffRed + 16u; // [0..3] Gram stages, [4] the update buffer, [5..8] Gram stages read
+constexpr unsigned kNBars = 9u;
+constexpr unsigned kNSmemDoubles = kNOffBar + 10u;
 static_assert(2u * (kNSmemDoubles * sizeof(double) + 1024u) <= 228u * 1024u, "two CTAs per SM");
 inline size_t batchn_smem_bytes() { return (size_t)kNSmemDoubles * sizeof(double); }
+
+__device__ __forceinline__ void init_bars_n(uint64_t *const bars)
+{
+  for (unsigned b = 0u; b < kNBars; ++b)
+    mbar_init(&bars[b], (b < 5u) ? 1u : kGramWarps);
+  mbar_fence_init();
+}
+
+__device__ __forceinline__ void inval_bars_n(uint64_t *const bars)
+{
+  for (unsigned b = 0u; b < kNBars; ++b)
+    mbar_inval(&bars[b]);
+}
+
+// The Gram phase of a CTA of 4 warps over nt tiles, one per stage: issue(k) by a
+// lane of warp 3 into stage k mod 4 once the Gram warps have read tile k - 4,
+// add(k) by each Gram warp when tile k has landed.  1 if a wait gave up.
+template <typename I, typename A>
+__device__ __forceinline__ int gram_phase_n(uint64_t *const bars, const unsigned nt, const I &issue, const A &add)
+{
+  const unsigned tid = threadIdx.x, warp = tid >> 5;
+  int failed = 0;
+  if (tid == kNIssuer) {
+    for (unsigned k = 0u; k < nt && !failed; ++k) {
+      if (k >= kNGStages && !mbar_wait_bounded(&bars[5u + k % kNGStages], (k / kNGStages - 1u) & 1u, kWaitLimit))
+        failed = 1;
+      else
+        issue(k);
+    }
+  }
+  else if (warp < kGramWarps) {
+    for (unsigned k = 0u; k < nt && !failed; ++k) {
+      if (!__all_sync(0xffffffffu, mbar_wait_bounded(&bars[k % kNGStages], (k / kNGStages) & 1u, kWaitLimit)))
+        failed = 1;
+      else {
+        add(k);
+        __syncwarp();
+        if ((tid & 31u) == 0u)
+          mbar_arrive(&bars[5u + k % kNGStages]);
+      }
+    }
+  }
+  failed = __syncthreads_or(failed);
+  if (failed && tid == 0u) // the copies in flight land (bounded) before anything else
+    for (unsigned b = 0u; b < kNGStages; ++b)
+      for (unsigned par = 0u; par < 2u; ++par)
+        (void)mbar_wait_bounded(&bars[b], par, kWaitLimit / 8);
+  return failed;
+}
 
 template <bool SORT, bool ACCV>
 __device__ __forceinline__ void pair_step_n(const StepParams &P, const unsigned step, const unsigned pair,
@@ -1181,11 +1231,8 @@ __device__ __forceinline__ void pair_step_n(const StepParams &P, const unsigned 
 
   for (unsigned i = tid; i < 256u; i += kNThreads)
     reinterpret_cast<uint32_t *>(s0)[i] = reinterpret_cast<const uint32_t *>(P.strat0)[i];
-  if (tid == 0u) {
-    for (unsigned b = 0u; b < 5u; ++b)
-      mbar_init(&bars[b], 1u);
-    mbar_fence_init();
-  }
+  if (tid == 0u)
+    init_bars_n(bars);
   __syncthreads();
 
   pdl_wait(); // G, V and the counters are the launch before's
@@ -1202,31 +1249,12 @@ __device__ __forceinline__ void pair_step_n(const StepParams &P, const unsigned 
     tma_load_3d(st, &P.tmGram, 0, (int)k, (int)(iBlk * kNColB), &bars[s]);
     tma_load_3d(st + 16u * kGramColLd, &P.tmGram, 0, (int)k, (int)(jBlk * kNColB), &bars[s]);
   };
-  if (tid == kNIssuer)
-    for (unsigned k = 0u; k + 1u < kNGStages && k < ntile; ++k)
-      issue_gram(k);
-  unsigned k = 0u;
-  int failed = 0;
-  for (; k < ntile; ++k) {
-    if (tid == kNIssuer && k + kNGStages - 1u < ntile)
-      issue_gram(k + kNGStages - 1u); // into the stage released after tile k - 1
-    int fail = 0;
-    if (warp < GramShape<1u>::warps) {
-      if (!mbar_wait_bounded(&bars[k % kNGStages], (k / kNGStages) & 1u, kWaitLimit))
-        fail = 1;
-      else if (gl.on)
-        gacc.tile(stg + (k % kNGStages) * kGramTileLd, gl);
-    }
-    failed = __syncthreads_or(fail);
-    if (failed)
-      break;
-  }
-  if (failed) {
-    if (tid == 0u) { // the copies in flight land (bounded) before anything else, report
-      for (unsigned q = k; q < ntile && q < k + kNGStages; ++q)
-        (void)mbar_wait_bounded(&bars[q % kNGStages], (q / kNGStages) & 1u, kWaitLimit / 8);
+  if (gram_phase_n(bars, ntile, issue_gram, [&](const unsigned k) {
+        if (gl.on)
+          gacc.tile(stg + (k % kNGStages) * kGramTileLd, gl);
+      })) {
+    if (tid == 0u)
       atomicOr(P.err, kErrWaitTimeout);
-    }
     return;
   }
   gacc.put(gl, [&](const unsigned o, const double v) { R[o] = v; });
@@ -1333,8 +1361,8 @@ constexpr unsigned kN2OffRB = kN2OffVlA + 1024u;
 constexpr unsigned kN2OffVlB = kN2OffRB + 32u * kVTLd;
 constexpr unsigned kN2OffS0 = kN2OffVlB + 1024u;
 constexpr unsigned kN2OffRed = kN2OffS0 + 128u; // [0..3] A's counts, [4..7] B's, [8..9] flags
-constexpr unsigned kN2OffBar = kN2OffRed + 8u;  // [0..3] Gram stages, [4] the update buffer
-constexpr unsigned kN2SmemDoubles = kN2OffBar + 8u;
+constexpr unsigned kN2OffBar = kN2OffRed + 8u;  // as kNOffBar
+constexpr unsigned kN2SmemDoubles = kN2OffBar + 10u;
 static_assert(2u * (kN2SmemDoubles * sizeof(double) + 1024u) <= 228u * 1024u, "two CTAs per SM");
 inline size_t batchn2_smem_bytes() { return (size_t)kN2SmemDoubles * sizeof(double); }
 
@@ -1355,11 +1383,8 @@ __device__ __forceinline__ void pair_step2n(const StepParams &PA, const unsigned
 
   for (unsigned i = tid; i < 256u; i += kNThreads)
     reinterpret_cast<uint32_t *>(s0)[i] = reinterpret_cast<const uint32_t *>(PA.strat0)[i];
-  if (tid == 0u) {
-    for (unsigned b = 0u; b < 5u; ++b)
-      mbar_init(&bars[b], 1u);
-    mbar_fence_init();
-  }
+  if (tid == 0u)
+    init_bars_n(bars);
   __syncthreads();
 
   // ------------------------------ 1. Grams --------------------------------
@@ -1382,33 +1407,15 @@ __device__ __forceinline__ void pair_step2n(const StepParams &PA, const unsigned
     gacc.put(gl, [&](const unsigned o, const double v) { R[o] = v; });
     gacc.clear();
   };
-  if (tid == kNIssuer)
-    for (unsigned k = 0u; k + 1u < kNGStages && k < nt; ++k)
-      issue_gram(k);
-  unsigned k = 0u;
-  int failed = 0;
-  for (; k < nt; ++k) {
-    if (tid == kNIssuer && k + kNGStages - 1u < nt)
-      issue_gram(k + kNGStages - 1u);
-    int fail = 0;
-    if (warp < GramShape<1u>::warps) {
-      if (!mbar_wait_bounded(&bars[k % kNGStages], (k / kNGStages) & 1u, kWaitLimit))
-        fail = 1;
-      else if (gl.on)
-        gacc.tile(stg + (k % kNGStages) * kGramTileLd, gl);
-      if (k + 1u == ntA)
-        put_gram(sm + kN2OffRA);
-      else if (k + 1u == nt)
-        put_gram(sm + kN2OffRB);
-    }
-    failed = __syncthreads_or(fail);
-    if (failed)
-      break;
-  }
-  if (failed) {
+  if (gram_phase_n(bars, nt, issue_gram, [&](const unsigned k) {
+        if (gl.on)
+          gacc.tile(stg + (k % kNGStages) * kGramTileLd, gl);
+        if (k + 1u == ntA)
+          put_gram(sm + kN2OffRA);
+        else if (k + 1u == nt)
+          put_gram(sm + kN2OffRB);
+      })) {
     if (tid == 0u) {
-      for (unsigned q = k; q < nt && q < k + kNGStages; ++q)
-        (void)mbar_wait_bounded(&bars[q % kNGStages], (q / kNGStages) & 1u, kWaitLimit / 8);
       atomicOr(PA.err, kErrWaitTimeout);
       atomicOr(PB.err, kErrWaitTimeout);
     }
