@@ -5,7 +5,9 @@
 * ``build_strat`` -> gpujachx_b200/lib/strat.so   (the reference's pivot-pair tables,
                                                    compiled unchanged from its
                                                    strat/<family>/NNNNN.h headers,
-                                                   symbols "<family>%05u")
+                                                   symbols "<family>%05u"; without
+                                                   its tree the tables that a
+                                                   construction gives, fewer orders)
 * ``build_x1``    -> gpujachx_b200/lib/x1         (the x1 command line)
 * ``build_pp``    -> gpujachx_b200/lib/libgjx_pp.so (accuracy post-processor, host
                                                    code in x87 extended precision)
@@ -105,6 +107,21 @@ def build_pp(force: bool = False, verbose: bool = True) -> str:
     return PP
 
 
+# in a strategy library that was built without the reference tree
+STRAT_MARK = "gjx_constructed_tables"
+
+
+def strat_symbols() -> list[str]:
+    return subprocess.run(["nm", "-D", "--defined-only", STRAT], capture_output=True, text=True,
+                          check=True).stdout.split()[2::3]
+
+
+def strat_constructed() -> bool:
+    """Whether the strategy library was built without the reference tree, from
+    the constructions of strat_gen alone (fewer orders than the reference ships)."""
+    return STRAT_MARK in strat_symbols()
+
+
 def build_strat(ref_root: str | None = None, force: bool = False, verbose: bool = True) -> str:
     """Compile the reference's strategy-table headers, where they lie, into strat.so.
 
@@ -113,15 +130,17 @@ def build_strat(ref_root: str | None = None, force: bool = False, verbose: bool 
     does, with the same exported symbol names.  The rowcyc and colcyc tables
     of orders 960 and 1024, which the reference does not ship, are added by
     its doubling construction (strat_gen).  Without a reference tree the
-    families are built whole by strat_gen, for the orders it gives.
+    families are built whole by strat_gen, for the orders it gives; the orders
+    left out are reported, the library is marked, and a marked library is built
+    again once a tree is given.
     """
     ref_root = ref_root or os.environ.get("GJX_REF_ROOT", "")
     sdir = os.path.join(ref_root, "strat") if ref_root else ""
-    if not force and os.path.exists(STRAT):
-        return STRAT
     have_ref = bool(sdir) and os.path.isdir(sdir)
-    if not have_ref and os.path.exists(STRAT):
+    if not force and os.path.exists(STRAT) and not (have_ref and strat_constructed()):
         return STRAT
+    if not have_ref and os.path.exists(STRAT) and not strat_constructed():
+        return STRAT  # the reference's tables are not replaced by fewer
     os.makedirs(LIBDIR, exist_ok=True)
     work = tempfile.mkdtemp(prefix="gjx_strat_")
     try:
@@ -152,7 +171,12 @@ def build_strat(ref_root: str | None = None, force: bool = False, verbose: bool 
                 objs = list(ex.map(one, STRAT_FAMILIES))
                 objs += list(ex.map(ext, sorted(strat_gen.extension_sources(sdir).items())))
             else:
-                objs = list(ex.map(ext, sorted(strat_gen.family_sources().items())))
+                mark = 'const char %s __attribute__((visibility("default"))) = 1;\n' % STRAT_MARK
+                objs = list(ex.map(ext, sorted(strat_gen.family_sources().items()) + [("mark.c", mark)]))
+                print("strat.so: no reference tree (GJX_REF_ROOT), so only the tables that a construction gives: "
+                      + strat_gen.CONSTRUCTED + ".  Other orders that the reference ships are left out "
+                      "(init_strats refuses them); the library is built again once the tree is given.",
+                      file=sys.stderr)
         tmp = STRAT + ".tmp"
         _run(["gcc", "-shared", "-o", tmp] + objs, verbose)
         os.replace(tmp, STRAT)

@@ -148,6 +148,11 @@ def modulus_table(n: int) -> np.ndarray:
     return np.array(steps, dtype=np.int64)
 
 
+# what family_tables gives, for messages
+CONSTRUCTED = ("mmstep and BrentL of orders 16, 32, ..., 896; rowcyc, colcyc, cycwor and cycloc of orders 2^k b, "
+               "b = 2, 6, 10, 14, 18, up to 896 (rowcyc and colcyc also 1024)")
+
+
 def family_tables():
     """(family, n, table) of every table that is built without a reference tree."""
     orders = sorted(b << k for b in (2, 6, 10, 14, 18) for k in range(10) if b << k <= 1024)

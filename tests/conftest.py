@@ -48,3 +48,18 @@ def load_golden(variant="base"):
         return None
     with open(p) as f:
         return json.load(f)
+
+
+def need_reference_tables():
+    """Skip where strat.so was built without the reference tree."""
+    from gpujachx_b200 import build as B
+    if B.strat_constructed():
+        pytest.skip("strat.so was built without the reference tree: not the reference's set of tables")
+
+
+def need_table(family, n):
+    """Skip where strat.so was built without the reference tree and has no such table."""
+    from gpujachx_b200 import build as B
+    name = "%s%05u" % (family, n)
+    if B.strat_constructed() and name not in B.strat_symbols():
+        pytest.skip(name + ": strat.so was built without the reference tree, and no construction gives this order")

@@ -9,11 +9,14 @@ an ulp."""
 import numpy as np
 import pytest
 
+from conftest import need_table
+
 pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("fam,n", [("rowcyc", 16384), ("colcyc", 15360)])
 def test_orthogonal_input_at_the_largest_orders(built, fam, n):
+    need_table(fam, n // 16)
     import torch
     import gpujachx_b200 as g
     g.init_strats(None, "cycwor", 32, fam, n // 16)

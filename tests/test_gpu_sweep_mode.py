@@ -7,6 +7,7 @@ import numpy as np
 import pytest
 
 from gpujachx_b200 import synth
+from conftest import need_table
 
 
 @pytest.mark.gpu
@@ -61,11 +62,12 @@ def test_cluster_sizes_give_the_same_bits(built, m, n, p, alg):
 @pytest.mark.gpu
 @pytest.mark.parametrize("m,n,p,alg,gen", [(256, 256, 256, 9, "svd_synth"), (1024, 480, 200, 11, "graded"),
                                            (2048, 1024, 512, 3, "graded"), (640, 640, 640, 1, "gaussian"),
-                                           (512, 256, 0, 11, "gaussian")])
+                                           (512, 256, 0, 11, "gaussian"), (1024, 288, 100, 11, "graded")])
 def test_two_pairs_per_cta_give_the_same_bits(built, m, n, p, alg, gen):
     """One CTA per block pair, per-step launches: two pairs per CTA (the form
-    used when a step has more pairs than SMs; 480 columns: 15 pairs per step,
-    the last one alone) against one."""
+    used when a step has more pairs than SMs; 480 and 288 columns: 15 and 9 pairs
+    per step, the last one alone) against one."""
+    need_table("cycwor", n // 16)
     import gpujachx_b200 as g
     kw = {"smin": 1e-8} if gen == "svd_synth" else {}
     G = synth.make(gen, m, n, 79, **kw)

@@ -13,6 +13,7 @@ import numpy as np
 import pytest
 
 from gpujachx_b200 import strat_gen
+from conftest import need_reference_tables, need_table
 
 
 def _load(oracle, strat_path, fam, n):
@@ -21,6 +22,7 @@ def _load(oracle, strat_path, fam, n):
 
 @pytest.mark.parametrize("fam", strat_gen.FAMILIES)
 def test_doubling_reproduces_every_shipped_table(fam, oracle, strat_path):
+    need_reference_tables()
     matched = 0
     for n in range(2, 449, 2):
         try:
@@ -35,6 +37,7 @@ def test_doubling_reproduces_every_shipped_table(fam, oracle, strat_path):
 @pytest.mark.parametrize("fam", strat_gen.FAMILIES)
 @pytest.mark.parametrize("n", strat_gen.ORDERS)
 def test_added_tables_are_the_doubling(fam, n, oracle, strat_path):
+    need_table(fam, n)
     got = _load(oracle, strat_path, fam, n)
     assert got.shape == (n - 1, n // 2, 2)
     assert np.array_equal(got, strat_gen.double_table(_load(oracle, strat_path, fam, n // 2), fam))
@@ -43,6 +46,7 @@ def test_added_tables_are_the_doubling(fam, n, oracle, strat_path):
 @pytest.mark.parametrize("fam", strat_gen.FAMILIES)
 @pytest.mark.parametrize("n", strat_gen.ORDERS)
 def test_added_tables_load_and_validate(fam, n, built):
+    need_table(fam, n)
     import gpujachx_b200 as g
     g.init_strats(None, "cycwor", 32, fam, n)
     info = g.strat_info()

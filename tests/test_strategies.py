@@ -11,6 +11,8 @@ import itertools
 import numpy as np
 import pytest
 
+from conftest import need_reference_tables
+
 FAMILIES = ("mmstep", "BrentL", "colcyc", "cycloc", "rowcyc", "cycwor")
 
 
@@ -28,6 +30,7 @@ def _orders(strat_path):
 
 
 def test_table_count(strat_path):
+    need_reference_tables()
     o = _orders(strat_path)
     # every shipped header (orders up to 896), and the rowcyc / colcyc tables
     # of orders 960 and 1024 that the build adds by the doubling construction
@@ -77,6 +80,7 @@ def test_strategy_ids(built):
 def test_validator_accepts_every_shipped_table(built):
     """gjx_validate_pairs on all tables (up to n1 = 1024): perfect matchings,
     full coverage; repeats only in mmstep (n/2 pairs twice, n steps)."""
+    need_reference_tables()
     import re
     import subprocess
     import gpujachx_b200 as g
