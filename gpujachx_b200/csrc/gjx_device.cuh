@@ -386,6 +386,13 @@ __device__ __forceinline__ void bar_sync(const unsigned id, const unsigned nthre
 __device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
+// A CTA's shared memory may be accessed from its cluster once the CTA has
+// started: every thread of every CTA arrives when it runs, and waits before the
+// cluster's first remote store.  No data is handed over (relaxed).  Between the
+// two lies the Gram phase, so nobody is waited for in practice.
+__device__ __forceinline__ void cluster_started() { asm volatile("barrier.cluster.arrive.relaxed;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait_started() { asm volatile("barrier.cluster.wait;" ::: "memory"); }
+
 // ---------------------------------------------------------------------------
 // mbarrier + bulk-copy (TMA engine) helpers, with bounded waits
 // ---------------------------------------------------------------------------

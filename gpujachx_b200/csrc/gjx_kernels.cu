@@ -215,6 +215,10 @@ __global__ void __launch_bounds__(kThreads, 1) l1_sweep_kernel(const __grid_cons
   uint64_t *const bars = reinterpret_cast<uint64_t *>(sm + kOffBar);
   const unsigned rank = (NSPLIT > 1u) ? (blockIdx.x % NSPLIT) : 0u;
   const unsigned pair = blockIdx.x / NSPLIT;
+  if (NSPLIT > 1u) { // agree[] below is the cluster's first remote store
+    cluster_started();
+    cluster_wait_started();
+  }
   for (unsigned step = 0u; step < P.steps1; ++step) {
     const size_t pidx = ((size_t)step * P.pairs + pair) * 2u;
     const unsigned iB = P.strat1[pidx + 0u], jB = P.strat1[pidx + 1u];

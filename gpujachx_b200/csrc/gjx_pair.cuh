@@ -674,6 +674,8 @@ __device__ __forceinline__ void pair_step(const StepParams &P, const unsigned st
   if (tid == 0u)
     init_bars(bars);
   __syncthreads();
+  if (NSPLIT > 1u)
+    cluster_started();
   pdl_wait(); // G, V and the counters are the launch before's
 
   int failed = 0;
@@ -741,6 +743,8 @@ __device__ __forceinline__ void pair_step(const StepParams &P, const unsigned st
     atomicOr(P.err, kErrWaitTimeout);
   }
   // our share of the lower triangle, into our R and the other CTAs' R
+  if (NSPLIT > 1u)
+    cluster_wait_started();
   {
     cg::cluster_group cl = cg::this_cluster();
     gacc.put(gl, [&](const unsigned o, const double v) {
