@@ -185,19 +185,24 @@ int upload_strat(DevCtx &ctx, const cudaStream_t st)
   return 0;
 }
 
-// the transforms of a step of the loaded outer table (and their flags)
-int ensure_vt(DevCtx &ctx)
+// the transforms of a step of the loaded outer table (and their flags), for the
+// calls that use them; false when the device has no memory for them
+bool ensure_vt(DevCtx &ctx)
 {
   const size_t pairs = g_strat.pairs1;
   if (pairs <= ctx.vt_pairs)
-    return 0;
+    return true;
   if (ctx.d_vt)
-    GJX_CUDA(cudaFree(ctx.d_vt), "cudaFree(transforms)");
+    (void)cudaFree(ctx.d_vt);
   ctx.d_vt = nullptr;
   ctx.vt_pairs = 0u;
-  GJX_CUDA(cudaMalloc(&ctx.d_vt, pairs * (gjx::kTransform * sizeof(double) + sizeof(unsigned))), "cudaMalloc(transforms)");
+  if (cudaMalloc(&ctx.d_vt, pairs * (gjx::kTransform * sizeof(double) + sizeof(unsigned))) != cudaSuccess) {
+    (void)cudaGetLastError();
+    ctx.d_vt = nullptr;
+    return false;
+  }
   ctx.vt_pairs = pairs;
-  return 0;
+  return true;
 }
 
 double secs(const clk::time_point a, const clk::time_point b)
@@ -210,14 +215,15 @@ double secs(const clk::time_point a, const clk::time_point b)
 // configured the kernels on this device and provides the device-side
 // working memory: the strategy tables d_s0 / d_s1 (uploaded) and two
 // 64-bit words d_cnt (counter, error word), plus a host mirror h_cnt of
-// those two words; d_ver (1024 words) and d_vt (ensure_vt), or null: no
-// launch per sweep, no update launches.  Nothing is allocated here (profiling events aside,
-// with prof).
+// those two words; d_ver (1024 words), or null: no launch per sweep; vt, the
+// context whose transforms the update launches use, or null: none.  Nothing
+// is allocated here (profiling events aside, with prof, and the transforms of
+// vt, without which the step kernels update).
 int run_sweeps_core(const unsigned routine, const unsigned nrow, const unsigned ncol, const unsigned nplus,
                     double *const dG, const unsigned lddG, double *const dV, const unsigned lddV, double *const dD,
                     const cudaStream_t st, const uint8_t *const d_s0, const uint16_t *const d_s1,
                     unsigned long long *const d_cnt, unsigned long long *const h_cnt, unsigned *const d_ver,
-                    double *const d_vt, const bool prof,
+                    DevCtx *const vt, const bool prof,
                     unsigned *const glbSwp, unsigned long long *const glb_s, unsigned long long *const glb_b)
 {
   const bool cdsort = (routine & GJX_CDSORT_1) != 0u, full = (routine & GJX_FULL_SVD) != 0u,
@@ -294,13 +300,13 @@ int run_sweeps_core(const unsigned routine, const unsigned nrow, const unsigned 
   // / without: 3072^2 (16 stages against 24) 323 / 372, 4864^2 without V (20
   // against 38) 1187 / 1511, 16384x256 (4 against 9) 23.1 / 24.7; but 4096x2048
   // (11 against 12) 146 / 141, HSVD 2048x1024 (3 against 3) 30.4 / 28.1
-  if (d_vt && !one_launch && !p.variant && !g_pairs_per_cta) {
+  if (vt && !one_launch && !p.variant && !g_pairs_per_cta) {
     const unsigned nst = (nrow + 255u) / 256u + (full ? (ncol + 255u) / 256u : 0u);
     const unsigned own = (p.width == 2u) ? 2u * nst : (nst + p.split - 1u) / p.split;
     const unsigned dealt = (p.pairs * nst + p.sms - 1u) / p.sms;
-    if (dealt + kUpdateMargin < own) {
-      p.vt = d_vt;
-      p.vflag = reinterpret_cast<unsigned *>(d_vt + (size_t)p.pairs * gjx::kTransform);
+    if (dealt + kUpdateMargin < own && ensure_vt(*vt)) {
+      p.vt = vt->d_vt;
+      p.vflag = reinterpret_cast<unsigned *>(p.vt + (size_t)p.pairs * gjx::kTransform);
       if (p.width == 2u)
         p.width = gjx::kWidthHalf;
     }
@@ -386,10 +392,8 @@ int run_sweeps(const unsigned routine, const unsigned nrow, const unsigned ncol,
     return r;
   if (const int r = upload_strat(*ctx, st))
     return r;
-  if (const int r = ensure_vt(*ctx))
-    return r;
   return run_sweeps_core(routine, nrow, ncol, nplus, dG, lddG, dV, lddV, dD, st, ctx->d_s0, ctx->d_s1, ctx->d_cnt,
-                         ctx->h_cnt, ctx->d_ver, ctx->d_vt, g_prof.on, glbSwp, glb_s, glb_b);
+                         ctx->h_cnt, ctx->d_ver, ctx, g_prof.on, glbSwp, glb_s, glb_b);
 }
 
 // argument checks of 1/HypJacL2.cu:39-77, same codes in the same order
@@ -1490,8 +1494,6 @@ int gjx_autotune(const unsigned routine, const unsigned nrow, const unsigned nco
     return r;
   if (const int r = upload_strat(*ctx, nullptr))
     return r;
-  if (const int r = ensure_vt(*ctx))
-    return r;
   const bool full = (routine & GJX_FULL_SVD) != 0u;
   const unsigned ld = nrow + (nrow & 1u);
   double *mem = nullptr;
@@ -1531,7 +1533,7 @@ int gjx_autotune(const unsigned routine, const unsigned nrow, const unsigned nco
           break;
         }
         rc = run_sweeps_core(routine, nrow, ncol, nplus, g, ld, full ? v : nullptr, ncol, d, nullptr, ctx->d_s0,
-                             ctx->d_s1, ctx->d_cnt, ctx->h_cnt, ctx->d_ver, ctx->d_vt, false, &swp, &s_, &b_);
+                             ctx->d_s1, ctx->d_cnt, ctx->h_cnt, ctx->d_ver, ctx, false, &swp, &s_, &b_);
         if (!rc && (cudaEventRecord(e1, nullptr) != cudaSuccess || cudaEventSynchronize(e1) != cudaSuccess ||
                     cudaEventElapsedTime(&ms, e0, e1) != cudaSuccess))
           rc = GJX_ERR_CUDA;

@@ -1,0 +1,88 @@
+"""Calls with no device memory left: what a faster route would take beside the
+caller's own buffers is not a condition of the call, which takes the route
+without it and gives the same bits."""
+
+import ctypes
+
+import numpy as np
+import pytest
+
+from gpujachx_b200 import synth
+
+pytestmark = pytest.mark.gpu
+
+
+class Full:
+    """The device's memory taken down to pieces of 64 KB, but for `hole` bytes."""
+
+    def __init__(self, hole=0):
+        import torch  # loads the CUDA runtime
+        torch.cuda.synchronize()
+        torch.cuda.empty_cache()
+        self.rt, self.hole, self.held = ctypes.CDLL("libcudart.so.12"), hole, []
+
+    def take(self, size):
+        p = ctypes.c_void_p()
+        if self.rt.cudaMalloc(ctypes.byref(p), ctypes.c_size_t(size)):
+            self.rt.cudaGetLastError()
+            return False
+        self.held.append(p)
+        return True
+
+    def __enter__(self):
+        if self.hole:
+            assert self.take(self.hole)
+        for k in range(37, 15, -1):
+            while self.take(1 << k):
+                pass
+        if self.hole:
+            self.rt.cudaFree(self.held.pop(0))
+        return self
+
+    def __exit__(self, *a):
+        for p in self.held:
+            self.rt.cudaFree(p)
+
+
+def _dev(G, full):
+    import torch
+    n = G.shape[1]
+    dG = torch.tensor(np.ascontiguousarray(G.T), device="cuda")
+    dV = torch.zeros((n, n), dtype=torch.float64, device="cuda") if full else None
+    return dG, dV, torch.zeros(n, dtype=torch.float64, device="cuda")
+
+
+def _bits(t):
+    return None if t is None else t.cpu().numpy().view(np.uint64)
+
+
+@pytest.mark.parametrize("m,n,apart", [(2048, 1024, False), (6016, 640, True)])
+def test_update_launch(m, n, apart, built):
+    """The transforms of the separate update launch: not allocated by a call that
+    does not use them, and done without by one that would."""
+    import torch
+
+    import gpujachx_b200 as g
+    G = synth.make("gaussian", m, n, 9)
+    g.init_strats(None, "cycwor", 32, "cycwor", n // 16)
+    runs = []
+
+    def run(bufs):
+        g.profile(False)
+        r = g.hypJacL2_dev(11, bufs[0], n, bufs[1], bufs[2])
+        torch.cuda.synchronize()
+        runs.append((r, g.profile_read()["launches"] > 2 * (n // 16 - 1) * r[1], bufs))
+
+    run(_dev(G, True))
+    g.lib().gjx_set_pairs_per_cta(1)  # the step kernels update
+    run(_dev(G, True))
+    g.lib().gjx_set_pairs_per_cta(0)
+    bufs = _dev(G, True)
+    g.lib().gjx_release_cache()
+    with Full():
+        run(bufs)
+    run(_dev(G, True))
+    assert [a for _, a, _ in runs] == [apart, False, False, apart]
+    for r, _, b in runs[1:]:
+        assert r == runs[0][0]
+        assert all(np.array_equal(_bits(x), _bits(y)) for x, y in zip(b, runs[0][2]))
