@@ -1361,6 +1361,30 @@ template <typename T> int grow(T *&p, size_t &cap, const size_t n, const char *w
   return 0;
 }
 
+// what the update of V on the side stream needs: two steps' V_loc, the stream
+// and its events; false when the device has no room for them (V is then
+// updated with G)
+bool side_ready(SplitCtx &c, const size_t vloc)
+{
+  cudaError_t e = cudaSuccess;
+  if (vloc > c.vloc_cap) {
+    (void)cudaFree(c.d_vloc);
+    c.d_vloc = nullptr;
+    c.vloc_cap = 0u;
+    e = cudaMalloc(&c.d_vloc, vloc * sizeof(double));
+    if (e == cudaSuccess)
+      c.vloc_cap = vloc;
+  }
+  if (e == cudaSuccess && !c.side)
+    e = cudaStreamCreateWithFlags(&c.side, cudaStreamNonBlocking);
+  for (cudaEvent_t *const ev : {&c.main_ev, &c.side_ev[0], &c.side_ev[1]})
+    if (e == cudaSuccess && !*ev)
+      e = cudaEventCreateWithFlags(ev, cudaEventDisableTiming);
+  if (e != cudaSuccess)
+    (void)cudaGetLastError();
+  return e == cudaSuccess;
+}
+
 // 2-D view (rows, columns) of a column-major matrix, box {128 rows, 32 columns}
 cudaError_t make_tile_map(CUtensorMap *tm, const double *base, const unsigned nrow, const unsigned ncol,
                           const unsigned ld)
@@ -1547,17 +1571,8 @@ int split_sweeps(const unsigned routine, const unsigned nrow, const unsigned nco
   const bool prof = profiling();
   const bool beside = full && !prof && p.pairs < p.sms &&
                       (size_t)p.pairs * p.tilesV * 8000u <=
-                          (size_t)(p.sms - p.pairs) * ((nrow + 63u) / 64u * 2500u + 130000u);
-  if (beside) {
-    if (const int r = grow(c.d_vloc, c.vloc_cap, 2u * (size_t)pairs * 4096u, "cudaMalloc(V_loc)"))
-      return r;
-    if (!c.side) {
-      SP_CUDA(cudaStreamCreateWithFlags(&c.side, cudaStreamNonBlocking), "side stream");
-      SP_CUDA(cudaEventCreateWithFlags(&c.main_ev, cudaEventDisableTiming), "event");
-      SP_CUDA(cudaEventCreateWithFlags(&c.side_ev[0], cudaEventDisableTiming), "event");
-      SP_CUDA(cudaEventCreateWithFlags(&c.side_ev[1], cudaEventDisableTiming), "event");
-    }
-  }
+                          (size_t)(p.sms - p.pairs) * ((nrow + 63u) / 64u * 2500u + 130000u) &&
+                      side_ready(c, 2u * (size_t)pairs * 4096u);
   // whatever way this function is left, the side stream's work is over
   struct Side {
     cudaStream_t s;

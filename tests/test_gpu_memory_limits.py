@@ -86,3 +86,35 @@ def test_update_launch(m, n, apart, built):
     for r, _, b in runs[1:]:
         assert r == runs[0][0]
         assert all(np.array_equal(_bits(x), _bits(y)) for x, y in zip(b, runs[0][2]))
+
+
+def test_split_form_v_beside(built):
+    """The two steps' V_loc of V's update on its own stream.  (A timed call
+    allocates the rest of the split form's memory for this order.)"""
+    import torch
+
+    import gpujachx_b200 as g
+    n = 4608  # 72 block pairs: more than any other call of the suite with V beside
+    G = np.asfortranarray(np.diag(np.logspace(0.0, -3.0, n)))
+    G[:2, :2] = [[1.0, 0.5], [0.25, 0.75]]
+    g.init_strats(None, "cycwor", 32, "cycwor", 64)
+    runs = []
+
+    def run(bufs):
+        r = g.hypJacL2_split(11, bufs[0], n, bufs[1], bufs[2])
+        torch.cuda.synchronize()
+        runs.append((r, g.profile_read()["launches"], bufs))
+
+    steps = n // 32 - 1
+    g.profile(True)
+    run(_dev(G, True))
+    g.profile(False)
+    bufs = _dev(G, True)
+    with Full():
+        run(bufs)
+    g.profile(False)
+    run(_dev(G, True))
+    assert [k for _, k, _ in runs] == [4 + c * steps * runs[0][0][1] for c in (2, 2, 4)]
+    for r, _, b in runs[1:]:
+        assert r == runs[0][0]
+        assert all(np.array_equal(_bits(x), _bits(y)) for x, y in zip(b, runs[0][2]))
