@@ -47,6 +47,13 @@ struct Strat {
 
 constexpr unsigned kUpdateMargin = 1u; // stages of 256 rows
 
+// The batched form's launch per sweep waits, in the kernel and with a limit of
+// 2e9 cycles, for up to 16 steps ahead of an item (a few pairs, all their steps
+// taken at once); a row of a pair takes 50 to 100 cycles a step, so the limit
+// would be met from about a million rows on.  Up to this many rows a wait stays
+// below a tenth of it; above, a step takes milliseconds and its launch nothing.
+constexpr unsigned kFlowRows = 1u << 17;
+
 std::mutex g_mtx;
 Strat g_strat;
 int g_verbose = 1;
@@ -646,8 +653,11 @@ int run_batch(const unsigned routine, const unsigned nmat, const unsigned *const
                                                           : gjx::kWidthHalf2;
   if (g_pairs_per_cta)
     width = g_pairs_per_cta;
-  // (very large batches: one launch per step, 36402 pairs 3745 against 3795)
-  int mode = (g_batch_mode >= 0) ? g_batch_mode : (items.size() <= 64u * (unsigned)sms) ? 1 : 0;
+  // (very large batches: one launch per step, 36402 pairs 3745 against 3795; and kFlowRows)
+  unsigned rows = 0u;
+  for (const unsigned b : order)
+    rows = std::max(rows, nrow[b]);
+  int mode = (g_batch_mode >= 0) ? g_batch_mode : (items.size() <= 64u * (unsigned)sms && rows <= kFlowRows) ? 1 : 0;
   {
     const auto t = g_batch_tuned.find(batch_key(nmat, nrow, ncol, nplus));
     if (t != g_batch_tuned.end()) {

@@ -146,7 +146,7 @@ void gjx_autotune_clear(void);
 
 /* The batched form's launches: -1 (default) the tuned choice
  * (gjx_autotune_batched), else one launch per sweep up to about ten thousand
- * block pairs per step and one per outer step index above; 0 one launch
+ * block pairs per step and 131072 rows and one per outer step index above; 0 one launch
  * per outer step index for the whole batch (every active matrix advances one
  * step), replayed from a CUDA graph; 1 one launch per sweep of the whole
  * batch, in which a CTA takes (matrix, step, pair) items in step order and

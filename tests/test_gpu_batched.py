@@ -105,3 +105,47 @@ def test_batch_autotuner_picks_and_keeps_bits(built):
         torch.cuda.synchronize()
         assert (res.sweeps[k], res.rot_s[k], res.rot_b[k]) == (sw, rs, rb)
         assert np.array_equal(_bits(batch[k][0]), _bits(dG)) and np.array_equal(_bits(batch[k][1]), _bits(dV))
+
+
+def _orthogonal(n, m):
+    """Column j of an m x n matrix: one entry, 2^-(j // 8)."""
+    import torch
+    G = torch.zeros((n, m), dtype=torch.float64, device="cuda")
+    s = torch.tensor([2.0 ** -(j // 8) for j in range(n)], dtype=torch.float64, device="cuda")
+    j = torch.arange(n, device="cuda")
+    G[j, j * (m // n)] = s
+    return G, s
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("m,launches", [(1 << 17, 2 * 4 + 1), ((1 << 17) + 64, 2 * 8 + 1)])
+def test_untuned_launches_by_rows(m, launches, built):
+    """One graph of 4 sweeps up to 2^17 rows, above it one of 8 steps (and initD)."""
+    import torch
+    import gpujachx_b200 as g
+    g.init_strats(None, "cycwor", 32, "cycwor", 4)
+    G, s = _orthogonal(64, m)
+    g.profile(False)
+    r = g.hypJacL2_batched(9, [G], [64], Ds=[torch.empty_like(s)])
+    torch.cuda.synchronize()
+    assert r.info == [0] and r.sweeps[0] == 1
+    assert g.profile_read()["launches"] == launches
+
+
+@pytest.mark.gpu
+def test_very_tall_matrix(built):
+    """8 block pairs of 4 M rows, 15 steps of about 0.1 s: in one launch per sweep
+    the last step's items would wait for the 14 before them, longer than a wait
+    may take."""
+    import torch
+    import gpujachx_b200 as g
+    g.init_strats(None, "cycwor", 32, "cycwor", 16)
+    G, s = _orthogonal(256, 1 << 22)
+    D = torch.zeros(256, dtype=torch.float64, device="cuda")
+    r = g.hypJacL2_batched(9, [G], [256], Ds=[D])
+    torch.cuda.synchronize()
+    assert r.info == [0] and r.sweeps[0] == 1 and r.rot_b[0] == 0
+    assert torch.equal(D, s * s)
+    assert torch.equal(G.amax(dim=1), torch.ones_like(s))
+    del G
+    torch.cuda.empty_cache()
