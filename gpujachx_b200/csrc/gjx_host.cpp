@@ -668,11 +668,15 @@ int run_batch(const unsigned routine, const unsigned nmat, const unsigned *const
     }
   }
   const unsigned cap = g_batch_cap ? g_batch_cap : gjx::kNSweep;
-  if (mode == 1) { // one launch per sweep (the dataflow form)
-    std::vector<uint32_t> fitems;
-    std::vector<uint16_t> fsteps;
-    std::vector<unsigned> vofs(nmat, 0u);
-    unsigned nver = 0u;
+  // the dataflow form's items, steps, block counts and their offsets; where the
+  // device has no memory for them a mode that was not asked for gives way
+  std::vector<uint32_t> fitems;
+  std::vector<uint16_t> fsteps;
+  std::vector<unsigned> vofs(nmat, 0u);
+  unsigned nver = 0u;
+  size_t f_steps = 0u, f_ver = 0u, f_vofs = 0u;
+  Free flow{nullptr};
+  if (mode == 1) {
     for (unsigned b = 0u; b < nmat; ++b)
       if (ok[b]) {
         vofs[b] = nver;
@@ -685,15 +689,23 @@ int run_batch(const unsigned routine, const unsigned nmat, const unsigned *const
             fitems.push_back((b << 16u) | q);
             fsteps.push_back((uint16_t)st1);
           }
-    const size_t f_items = 0u, f_steps = up(f_items + fitems.size() * 4u), f_ver = up(f_steps + fsteps.size() * 2u),
-                 f_vofs = up(f_ver + (size_t)nver * 4u), ftotal = up(f_vofs + (size_t)nmat * 4u);
-    char *fmem = nullptr;
-    GJX_CUDA(cudaMalloc(&fmem, ftotal), "cudaMalloc(batch flow)");
-    Free free_fmem{fmem};
-    auto *d_fitems = reinterpret_cast<uint32_t *>(fmem + f_items);
-    auto *d_fsteps = reinterpret_cast<uint16_t *>(fmem + f_steps);
-    auto *d_ver = reinterpret_cast<unsigned *>(fmem + f_ver);
-    auto *d_vofs = reinterpret_cast<unsigned *>(fmem + f_vofs);
+    f_steps = up(fitems.size() * 4u);
+    f_ver = up(f_steps + fsteps.size() * 2u);
+    f_vofs = up(f_ver + (size_t)nver * 4u);
+    const cudaError_t e = cudaMalloc(&flow.m, up(f_vofs + (size_t)nmat * 4u));
+    if (e == cudaErrorMemoryAllocation && g_batch_mode < 0) {
+      (void)cudaGetLastError();
+      flow.m = nullptr;
+      mode = 0;
+    }
+    else
+      GJX_CUDA(e, "cudaMalloc(batch flow)");
+  }
+  if (mode == 1) { // one launch per sweep (the dataflow form)
+    auto *d_fitems = reinterpret_cast<uint32_t *>(flow.m);
+    auto *d_fsteps = reinterpret_cast<uint16_t *>(flow.m + f_steps);
+    auto *d_ver = reinterpret_cast<unsigned *>(flow.m + f_ver);
+    auto *d_vofs = reinterpret_cast<unsigned *>(flow.m + f_vofs);
     GJX_CUDA(cudaMemcpyAsync(d_fitems, fitems.data(), fitems.size() * 4u, cudaMemcpyHostToDevice, st), "upload");
     GJX_CUDA(cudaMemcpyAsync(d_fsteps, fsteps.data(), fsteps.size() * 2u, cudaMemcpyHostToDevice, st), "upload");
     GJX_CUDA(cudaMemcpyAsync(d_vofs, vofs.data(), nmat * 4u, cudaMemcpyHostToDevice, st), "upload");

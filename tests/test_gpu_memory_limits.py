@@ -2,6 +2,7 @@
 caller's own buffers is not a condition of the call, which takes the route
 without it and gives the same bits."""
 
+import contextlib
 import ctypes
 
 import numpy as np
@@ -118,3 +119,28 @@ def test_split_form_v_beside(built):
     for r, _, b in runs[1:]:
         assert r == runs[0][0]
         assert all(np.array_equal(_bits(x), _bits(y)) for x, y in zip(b, runs[0][2]))
+
+
+def test_batched_form(built):
+    """The items of a launch per sweep: 6 bytes per block pair and step."""
+    import torch
+
+    import gpujachx_b200 as g
+    n, k = 4096, 24  # 128 pairs, 255 steps: 4.7 MB
+    g.init_strats(None, "cycwor", 32, "cycwor", n // 16)
+    s = torch.tensor([2.0 ** -(j // 64) for j in range(n)], dtype=torch.float64, device="cuda")
+    Gs = [torch.empty((n, n), dtype=torch.float64, device="cuda") for _ in range(k)]
+    Ds = [torch.zeros(n, dtype=torch.float64, device="cuda") for _ in range(k)]
+    launches = []
+    for full in (False, True):
+        for G, D in zip(Gs, Ds):
+            G.zero_().diagonal().copy_(s)
+            D.zero_()
+        g.profile(False)
+        with Full(hole=4 << 20) if full else contextlib.nullcontext():
+            r = g.hypJacL2_batched(9, Gs, n, Ds=Ds)
+            torch.cuda.synchronize()
+        launches.append(g.profile_read()["launches"])
+        assert r.info == [0] * k and r.sweeps == [1] * k
+        assert all(torch.equal(d, s * s) for d in Ds)
+    assert launches[0] == 2 * 4 + 1 and launches[1] == 2 * 256 + 1  # 4 sweeps a graph; 255 steps, 8 a graph
