@@ -271,6 +271,10 @@ int run_sweeps_core(const unsigned routine, const unsigned nrow, const unsigned 
     if (mode < 0)
       mode = tuned->second.second;
   }
+  // clusters of 8 have no launch per sweep: where one is asked for, the largest
+  // clusters that have one, unless 8 were asked for too
+  if (mode > 0 && d_ver && p.split == 8u)
+    p.split = gjx::l1_split(p.pairs, 0u);
   if (g_split && g_split * p.pairs <= 148u * 8u)
     p.split = g_split;
   // two block pairs per CTA: with 1 CTA per pair, when a step has more pairs

@@ -85,3 +85,27 @@ def test_two_pairs_per_cta_give_the_same_bits(built, m, n, p, alg, gen):
     assert (a.sweeps, a.rot_s, a.rot_b) == (b.sweeps, b.rot_s, b.rot_b)
     for x, y in ((a.U, b.U), (a.D, b.D)) + (((a.V, b.V),) if alg & 2 else ()):
         assert np.array_equal(x.view(np.uint64), y.view(np.uint64))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("m,n,split", [(2048, 256, 0), (1024, 512, 0), (4096, 64, 0), (2048, 256, 8)])
+def test_launch_per_sweep_of_few_pairs(built, m, n, split):
+    """Where a step's pairs would take clusters of 8 CTAs, which are launched per
+    step, a launch per sweep that is asked for takes clusters of 4; 8 asked for stay."""
+    import gpujachx_b200 as g
+    G = synth.make("gaussian", m, n, 80)
+    g.init_strats(None, "cycwor", 32, "cycwor", n // 16)
+    runs = []
+    for mode in (-1, 1):
+        g.lib().gjx_set_sweep_mode(mode)
+        g.lib().gjx_set_split(split if mode == 1 else 0)
+        g.profile(False)
+        r = g.hypJacL2(11, G, n)
+        runs.append((r, g.profile_read()["launches"]))
+    g.lib().gjx_set_split(0)
+    g.lib().gjx_set_sweep_mode(-1)
+    (a, _), (b, launches) = runs
+    assert launches == 2 + b.sweeps * (1 if split != 8 else n // 16 - 1)  # and initV, initD
+    assert (a.sweeps, a.rot_s, a.rot_b) == (b.sweeps, b.rot_s, b.rot_b)
+    for x, y in ((a.U, b.U), (a.D, b.D), (a.V, b.V)):
+        assert np.array_equal(x.view(np.uint64), y.view(np.uint64))
