@@ -655,6 +655,24 @@ int run_batch(const unsigned routine, const unsigned nmat, const unsigned *const
   unsigned width = (items.size() <= 2u * (unsigned)sms)   ? 1u
                    : (items.size() <= 8u * (unsigned)sms) ? gjx::kWidthHalf
                                                           : gjx::kWidthHalf2;
+  // Between one and two pairs per SM the SMs' work may take longer than the
+  // longest chain.  A pair costs its rows of G (and half of V's) and serial phases
+  // worth 1500; two on an SM take 1.05 times as long as one as far as that is
+  // serial, 2.2 times as far as it is rows.  ms, pairs: before / 1 / 3 -- 37 of 256 x 256,
+  // 296: 10.9 / 12.1 / 8.5; 26 of 256 x 256, 208: 10.8 / 9.0 / 8.0; 20, 160: 10.7 / 7.2 / 8.0; 30
+  // of 64..512, 256: 25.5 / 19.5 / 21.3; 36 of 2048 x 256, 288: 29.6 / 28.0 / 24.0; 72 of
+  // 16384 x 128, 288: 69.4 / 63.7 / 67.6.
+  if (items.size() > (unsigned)sms && items.size() <= 2u * (unsigned)sms) {
+    double all = 0.0, rows = 0.0, chain = 0.0;
+    for (const unsigned b : order) {
+      const double r = nrow[b] + (full ? 0.5 * ncol[b] : 0.0), n = mats[b].steps1;
+      rows += n * mats[b].p.pairs * r;
+      all += n * mats[b].p.pairs * (r + 1500.0);
+      chain = std::max(chain, n * (r + 1500.0));
+    }
+    if (all > sms * chain * (1.05 + 1.15 * rows / all))
+      width = gjx::kWidthHalf;
+  }
   if (g_pairs_per_cta)
     width = g_pairs_per_cta;
   // (very large batches: one launch per step, 36402 pairs 3745 against 3795; and kFlowRows)

@@ -115,7 +115,7 @@ void gjx_set_split(unsigned n);
  * 4 (batched form only: two block pairs per CTA of 4 warps, two such CTAs
  * per SM; the two pairs' serial phases run concurrently on 2 warps each), or
  * 0 (default): automatic -- the batched autotuner's
- * choice, else 1, 3 or 4 by the batch's block pairs per step
+ * choice, else 1, 3 or 4 by the batch's block pairs per step and their rows
  * (gjx_hypJacL2_batched), and in the per-step launches of a single matrix with one CTA per block pair when a
  * step has more block pairs than the GPU has SMs (one wave of CTAs instead of
  * two); else 1.  The results are the same bits for every value. */

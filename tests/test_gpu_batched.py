@@ -149,3 +149,33 @@ def test_very_tall_matrix(built):
     assert torch.equal(G.amax(dim=1), torch.ones_like(s))
     del G
     torch.cuda.empty_cache()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("m,n,count", [(64, 64, 148), (128, 128, 65), (256, 256, 20), (256, 256, 37), (512, 512, 18),
+                                       (4096, 128, 72)])
+def test_untuned_is_not_slower_than_two_pairs_per_cta(m, n, count, built):
+    """One to two block pairs per SM: a second wave of one-pair CTAs was up to 17 %
+    slower than two pairs per CTA, one launch per step.  (Measured 8 to 33 %
+    faster; the best of five runs of each.)"""
+    import time
+
+    import torch
+    import gpujachx_b200 as g
+    g.init_strats(None, "cycwor", 32, "cycwor", 4)
+    torch.manual_seed(6)
+    G = torch.randn((count, n, m), dtype=torch.float64, device="cuda")
+    W, D = torch.empty_like(G), torch.zeros((count, n), dtype=torch.float64, device="cuda")
+    best = {}
+    for _ in range(5):
+        for form in ((0, -1), (2, 0)):
+            g.lib().gjx_set_pairs_per_cta(form[0])
+            g.lib().gjx_set_batch_mode(form[1])
+            W.copy_(G)
+            torch.cuda.synchronize()
+            t = time.perf_counter()
+            g.hypJacL2_batched(9, list(W), n, Ds=list(D))
+            best[form] = min(best.get(form, 1e9), time.perf_counter() - t)
+    g.lib().gjx_set_pairs_per_cta(0)
+    g.lib().gjx_set_batch_mode(-1)
+    assert best[0, -1] < best[2, 0]
