@@ -1567,9 +1567,11 @@ int split_sweeps(const unsigned routine, const unsigned nrow, const unsigned nco
   // kernel takes (tiles of 8 K cycles against 2.5 K cycles per 64 rows of the
   // Gram products and 130 K of the rest), else it would delay the next update.
   // ms per call, beside / in one launch with G's: 4096^2 346 / 422 (64 CTAs of the
-  // pair kernel), HSVD 1600x1344 59.4 / 62.0.
+  // pair kernel), HSVD 1600x1344 59.4 / 62.0; 16384x5120 (80) 122 / 137 a sweep, but
+  // 5120^2 is over the line.  A sweep of one step (64 columns) has no next pair
+  // kernel before the host's turn: 256x64 253 / 240 us.
   const bool prof = profiling();
-  const bool beside = full && !prof && p.pairs < p.sms &&
+  const bool beside = full && !prof && c.steps1 > 1u && p.pairs < p.sms &&
                       (size_t)p.pairs * p.tilesV * 8000u <=
                           (size_t)(p.sms - p.pairs) * ((nrow + 63u) / 64u * 2500u + 130000u) &&
                       side_ready(c, 2u * (size_t)pairs * 4096u);

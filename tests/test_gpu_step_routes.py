@@ -77,13 +77,17 @@ def test_update_launch_with_unchanged_pairs(built):
     _same(g.hypJacL2(10, G, n), ref, True)
 
 
-@pytest.mark.parametrize("m,n,nplus,alg", [(64, 64, 64, 11), (1088, 320, 100, 11), (2112, 2048, 2048, 3), (512, 512, 512, 10)])
-def test_split_form_with_v_beside(m, n, nplus, alg, built):
-    """Timed (gjx_profile) launches keep V's update on the main stream."""
+@pytest.mark.parametrize("m,n,nplus,alg,beside", [(64, 64, 64, 11, False), (1088, 320, 100, 11, True), (2112, 2048, 2048, 3, True),
+                                                  (512, 512, 512, 10, True), (192, 128, 60, 11, True),
+                                                  (5120, 5120, 5120, 10, False)])
+def test_split_form_with_v_beside(m, n, nplus, alg, beside, built):
+    """Timed (gjx_profile) launches keep V's update on the main stream: two
+    launches a step, with V beside four (and initV, the maxima of V and of G,
+    initD).  Not beside: one step a sweep, and too little room beside 80 pairs."""
     import torch
 
     import gpujachx_b200 as g
-    G = synth.make("graded" if nplus < n else "gaussian", m, n, 8)
+    G = synth.make("graded" if nplus < n else "gaussian", m, n, 8) if n < 5120 else np.diag(np.logspace(0.0, -4.0, n))
     g.init_strats(None, "cycwor", 32, "cycwor", n // 16)
     runs = []
     for timed in (True, False):
@@ -92,6 +96,8 @@ def test_split_form_with_v_beside(m, n, nplus, alg, built):
         dD = torch.zeros(n, dtype=torch.float64, device="cuda")
         g.profile(timed)
         counts = g.hypJacL2_split(alg, dG, nplus, dV, dD)
+        per_step = 4 if beside and not timed else 2
+        assert g.profile_read()["launches"] == 4 + per_step * (n // 32 - 1) * counts[1]
         g.profile(False)
         runs.append((counts, dG.cpu().numpy(), dV.cpu().numpy(), dD.cpu().numpy()))
     a, b = runs
