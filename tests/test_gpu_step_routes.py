@@ -62,8 +62,9 @@ def test_update_launch(m, n, nplus, alg, built):
 
 
 def test_update_launch_with_unchanged_pairs(built):
-    """Blocks orthogonal to each other, some of them orthogonal within: most
-    pairs keep their columns (ALG 10 does not sort)."""
+    """Blocks orthogonal to each other (ALG 10 does not sort).  In some each column
+    has one entry, in a row of its own: their Gram matrices are diagonal, so a
+    pair of two of them rotates nothing and its flag is clear."""
     import gpujachx_b200 as g
     m, n = 8192, 640
     r = np.random.default_rng(4)
@@ -71,10 +72,19 @@ def test_update_launch_with_unchanged_pairs(built):
     for b in range(n // 16):
         blk = r.standard_normal((m // 64, 16))
         G[b * (m // 64):(b + 1) * (m // 64), 16 * b:16 * b + 16] = blk if b % 5 == 0 else np.linalg.qr(blk)[0] * 2.0 ** (b % 7)
+        if b % 5 > 2:
+            G[:, 16 * b:16 * b + 16] = 0.0
+            G[b * (m // 64) + np.arange(16), 16 * b + np.arange(16)] = 3.0 * 2.0 ** (np.arange(16) % 3)
     g.init_strats(None, "cycwor", 32, "cycwor", n // 16)
     ref = _fused(g, 10, G, n)
     g.lib().gjx_set_sweep_mode(-1)
-    _same(g.hypJacL2(10, G, n), ref, True)
+    g.profile(False)
+    r = g.hypJacL2(10, G, n)
+    assert g.profile_read()["launches"] > 2 * (n // 16 - 1) * r.sweeps  # two launches a step
+    _same(r, ref, True)
+    keep = np.flatnonzero(np.arange(n) // 16 % 5 > 2)  # the columns of those blocks
+    assert np.array_equal(r.U[:, keep], (G[:, keep] != 0.0).astype(float))
+    assert np.array_equal(r.V[:, keep], np.eye(n)[:, keep])
 
 
 @pytest.mark.parametrize("m,n,nplus,alg,beside", [(64, 64, 64, 11, False), (1088, 320, 100, 11, True), (2112, 2048, 2048, 3, True),
