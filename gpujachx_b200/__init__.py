@@ -33,7 +33,7 @@ STRATEGIES = ("mmstep", "BrentL", "colcyc", "cycloc", "rowcyc", "cycwor")
 # exported by libgjx.so, as declared in include/gjx.h
 EXPORTS = ("hypJacL2", "init_strats", "gjx_init_strats", "gjx_strat_info", "gjx_get_strat1",
            "gjx_hypJacL2_dev", "gjx_release_cache", "gjx_set_verbose", "gjx_last_error",
-           "gjx_version", "gjx_rsqrt_rn_dev", "gjx_profile", "gjx_profile_read", "gjx_hypJacL2_noalloc",
+           "gjx_version", "gjx_rsqrt_rn_dev", "gjx_exact_ops_dev", "gjx_profile", "gjx_profile_read", "gjx_hypJacL2_noalloc",
            "gjx_validate_pairs", "gjx_validate_strats", "gjx_configure_device", "gjx_h5_read", "gjx_h5_write",
            "gjx_hypJacL2_batched", "gjx_set_sweep_mode", "gjx_set_split", "gjx_set_pairs_per_cta", "gjx_autotune",
            "gjx_autotune_clear", "gjx_wait_selftest")
@@ -89,6 +89,8 @@ def lib() -> ctypes.CDLL:
     L.gjx_version.restype = ctypes.c_char_p
     L.gjx_rsqrt_rn_dev.argtypes = [ctypes.c_void_p, ctypes.c_void_p, u]
     L.gjx_rsqrt_rn_dev.restype = i
+    L.gjx_exact_ops_dev.argtypes = [u] + [ctypes.c_void_p] * 4 + [u]
+    L.gjx_exact_ops_dev.restype = i
     L.gjx_profile.argtypes = [i]
     L.gjx_profile.restype = None
     L.gjx_profile_read.argtypes = [pull, pull, pd]

@@ -205,6 +205,18 @@ __device__ __forceinline__ double sqrt_try(const double x, bool &ok)
   return s;
 }
 
+// 1 / sqrt(f), f = 1 +- t^2, by g = 1 - f (exact) for |g| < 2^-30: 1 + g (1/2 +
+// 3/8 g) rounded once.  There 1 + g/2 is a representable number, a midpoint or a
+// quarter of the spacing, and the true value lies above it by 3/8 g^2 + ...: the
+// computed sum lies above it too (1/2 is taken one ulp larger, for the g whose
+// 3/8 g is lost) and by less than a quarter of the spacing, so it rounds as the
+// true value does; for g < 0 1 + g/2 is representable and both round to it.
+__device__ __forceinline__ double rsqrt_near1(const double g, bool &ok)
+{
+  ok = hi_abs(g) < ((1023 - 30) << 20);
+  return __fma_rn(g, __fma_rn(0.375, g, 0x1.0000000000001p-1), 1.0);
+}
+
 // rsqrt_rn: the fast path, and rsqrt_rn_full for what it does not settle
 __device__ __forceinline__ bool rsqrt_range(const double a) // 2^-960 <= a < 2^960
 {
@@ -291,13 +303,6 @@ static __device__ __noinline__ RotRaw rot_ieee(const bool trig, const double Apq
 // against Dp Dq tol^2 (tol^2 = 2^-101 to 2^-52), without the two square roots:
 // the high words order as the rounded sides do when they differ by 2 or more
 // (2^-20 relatively, the roundings 2^-49).
-// The reciprocal root of f = 1 +- t^2 for g = 1 - f (exact), |g| < 2^-30, is
-// 1 + g (1/2 + 3/8 g) rounded once.  There 1 + g/2 is a representable number, a
-// midpoint or a quarter of the spacing, and the true value lies above it by
-// 3/8 g^2 + ...: the computed sum lies above it too (1/2 is taken one ulp larger,
-// for the g whose 3/8 g is lost) and by less than a quarter of the spacing, so
-// it rounds as the true value does; for g < 0 1 + g/2 is representable and
-// both round to it.
 // Measured (inner_rot, one warp; two warps per sub-partition): 451 and 538
 // cycles, against 715 and 775 with the IEEE operations one after the other.
 // bad: a value that this lane's rotation uses is not proved, or the test is
@@ -326,8 +331,8 @@ __device__ __forceinline__ RotRaw rot_try(const bool trig, const double Apq, con
   const double t = rcp_try(CT2 + ((small || large) ? alt : sq), ok_t);
   const double f = __fma_rn((!MIXED || trig) ? t : -t, t, 1.0), g = 1.0 - f;
   const double cr = rsqrt_try(f, ok_c);
-  const bool near1 = hi_abs(g) < ((1023 - 30) << 20);
-  const double c1 = near1 ? __fma_rn(g, __fma_rn(0.375, g, 0x1.0000000000001p-1), 1.0) : cr;
+  bool near1;
+  const double cn = rsqrt_near1(g, near1), c1 = near1 ? cn : cr;
   r.c = large ? 1.0 : (fixed ? kCoshIFix : c1);
   r.t = fixed ? kTanh1Fix : copysign(t, ct2);
   r.b = (unsigned long long)__double_as_longlong(r.c) != 0x3FF0000000000000ull; // c != 1

@@ -1346,6 +1346,15 @@ int gjx_release_cache(void)
   return 0;
 }
 
+int gjx_exact_ops_dev(const unsigned op, const double *h, const double *a, double *out, int *ok, const unsigned n)
+{
+  if (op > 4u)
+    return -1;
+  GJX_CUDA(gjx::launch_exact_ops_test(op, h, a, out, ok, n, nullptr), "exact operations");
+  GJX_CUDA(cudaStreamSynchronize(nullptr), "exact operations");
+  return 0;
+}
+
 int gjx_rsqrt_rn_dev(const double *in, double *out, const unsigned n)
 {
   GJX_CUDA(gjx::launch_rsqrt_test(in, out, n, nullptr), "rsqrt_rn");

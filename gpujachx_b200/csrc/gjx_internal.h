@@ -147,5 +147,7 @@ int family_tables(unsigned n0, unsigned n1, std::vector<uint8_t> &s0, unsigned &
 
 // exposed for the parity tests of the primitives
 cudaError_t launch_rsqrt_test(const double *in, double *out, unsigned n, cudaStream_t s);
+cudaError_t launch_exact_ops_test(unsigned op, const double *h, const double *a, double *out, int *ok, unsigned n,
+                                  cudaStream_t s);
 
 } // namespace gjx

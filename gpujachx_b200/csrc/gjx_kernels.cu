@@ -337,6 +337,32 @@ __global__ void rsqrt_test_kernel(const double *const in, double *const out, con
     out[i] = rsqrt_rn(in[i]);
 }
 
+__global__ void exact_ops_test_kernel(const unsigned op, const double *const h, const double *const a,
+                                      double *const out, int *const ok, const unsigned n)
+{
+  const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n)
+    return;
+  bool p;
+  switch (op) {
+  case 0u:
+    out[i] = div_try(h[i], a[i], p);
+    break;
+  case 1u:
+    out[i] = rcp_try(a[i], p);
+    break;
+  case 2u:
+    out[i] = sqrt_try(a[i], p);
+    break;
+  case 3u:
+    out[i] = rsqrt_try(a[i], p);
+    break;
+  default:
+    out[i] = rsqrt_near1(1.0 - a[i], p);
+  }
+  ok[i] = p ? 1 : 0;
+}
+
 // ---------------------------------------------------------------------------
 // launchers and tensor maps
 // ---------------------------------------------------------------------------
@@ -708,6 +734,13 @@ cudaError_t launch_wait_selftest(long long limit, int *timed_out, long long *cyc
 cudaError_t launch_fill_random(double *a, size_t n, unsigned long long seed, cudaStream_t s)
 {
   fill_random_kernel<<<1024u, 256u, 0, s>>>(a, n, seed);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_exact_ops_test(unsigned op, const double *h, const double *a, double *out, int *ok, unsigned n,
+                                  cudaStream_t s)
+{
+  exact_ops_test_kernel<<<(n + 255u) / 256u, 256u, 0, s>>>(op, h, a, out, ok, n);
   return cudaGetLastError();
 }
 

@@ -303,6 +303,13 @@ const char *gjx_version(void);
  * device arrays; returns 0 or GJX_ERR_CUDA. */
 int gjx_rsqrt_rn_dev(const double *in, double *out, const unsigned n);
 
+/* Device check of the operations of the rotations that prove their rounding:
+ * out[i] = h[i] / a[i] (op 0), 1 / a[i] (1), sqrt(a[i]) (2), 1 / sqrt(a[i])
+ * (3, and 4 by the series for a[i] next to 1); where ok[i] it is the value
+ * rounded to nearest (operands and results well within the normal range).
+ * Device arrays (h for op 0 only).  0, -1 (op) or GJX_ERR_CUDA. */
+int gjx_exact_ops_dev(unsigned op, const double *h, const double *a, double *out, int *ok, unsigned n);
+
 #ifdef __cplusplus
 }
 #endif

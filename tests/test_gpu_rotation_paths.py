@@ -75,3 +75,73 @@ def test_reciprocal_square_root_is_correctly_rounded(exponents, built, oracle):
     torch.cuda.synchronize()
     want = np.array([oracle.rsqrt_rn(v) for v in x])
     assert np.array_equal(out.cpu().numpy().view(np.uint64), want.view(np.uint64))
+
+
+def _significands(r, n):
+    """Random ones, few leading or trailing bits set, next to 1 and 2."""
+    m = r.integers(0, 1 << 52, n, dtype=np.uint64)
+    m[::7] &= np.uint64(0xF)
+    m[1::7] |= np.uint64((1 << 52) - 16)
+    m[2::7] &= ~np.uint64((1 << 40) - 1)
+    return 1.0 + m.astype(np.float64) * 2.0 ** -52
+
+
+def _midpoint(q):
+    """q + ulp(q) / 2, a float between two neighbours: as an exact fraction."""
+    from fractions import Fraction
+    return (Fraction(float(q)) + Fraction(float(np.nextafter(q, np.inf)))) / 2
+
+
+@pytest.mark.parametrize("op", [0, 1, 2, 3, 4])
+def test_proved_operations(op, built, oracle):
+    """What the branch-free quotient, reciprocal, roots and the series next to 1
+    declare proved is the IEEE operation's result (the correctly rounded
+    reciprocal root for the last two), on random operands and on operands whose
+    result lies as near to a midpoint of two floats as one operand can put it; and
+    they prove all but a few of the random ones."""
+    import torch
+
+    import gpujachx_b200 as g
+    r = np.random.default_rng(11 + op)
+    n, hard = 200000, 20000
+    e = r.integers(-300, 300, n) if op < 2 else 2 * r.integers(-300, 300, n) + r.integers(0, 2, n)
+    a = np.ldexp(_significands(r, n), e)
+    h = np.ldexp(_significands(r, n), r.integers(-300, 300, n)) * r.choice([-1.0, 1.0], n)
+    if op < 2:
+        a *= r.choice([-1.0, 1.0], n)
+    if op == 4:  # 1 +- t^2, t from 2^-60 to 2^-10 (proved below 2^-15)
+        t = np.ldexp(_significands(r, n), r.integers(-60, -10, n))
+        a = 1.0 + np.where(r.random(n) < 0.5, 1.0, -1.0) * t * t
+    else:
+        q = 1.0 + r.random(hard)
+        for i in range(hard):
+            m = _midpoint(q[i])
+            if op == 0:
+                h[i] = float(m * abs(_frac(a[i])))
+            elif op == 1:
+                a[i] = float(1 / m)
+            elif op == 2:
+                a[i] = float(m * m)
+            else:
+                a[i] = float(1 / (m * m))
+    dh, da = torch.from_numpy(h).cuda(), torch.from_numpy(a).cuda()
+    out, ok = torch.empty_like(da), torch.zeros(n, dtype=torch.int32, device="cuda")
+    assert g.lib().gjx_exact_ops_dev(op, dh.data_ptr(), da.data_ptr(), out.data_ptr(), ok.data_ptr(), n) == 0
+    out, ok = out.cpu().numpy(), ok.cpu().numpy() != 0
+    want = (h / a if op == 0 else 1.0 / a if op == 1 else np.sqrt(a) if op == 2 else
+            np.array([oracle.rsqrt_rn(v) for v in a]))
+    assert np.array_equal(out[ok].view(np.uint64), want[ok].view(np.uint64))
+    plain = np.arange(n) >= hard
+    if op == 4:
+        plain &= np.abs(1.0 - a) < 2.0 ** -30
+        assert ok[plain].all() and plain.sum() > n // 2
+        assert not ok[np.abs(1.0 - a) >= 2.0 ** -30].any()
+    else:
+        plain &= np.arange(n) % 7 > 2
+        assert ok[plain].mean() > 0.99
+    assert g.lib().gjx_exact_ops_dev(5, 0, 0, 0, 0, 0) == -1
+
+
+def _frac(x):
+    from fractions import Fraction
+    return Fraction(float(x))
