@@ -305,12 +305,17 @@ int run_sweeps_core(const unsigned routine, const unsigned nrow, const unsigned 
   // one launch per sweep when all clusters of a step are resident together
   bool one_launch = d_ver && mode > 0 && g_strat.n1 <= 1024u && gjx::sweep_kernel_fits(cdsort, full, p);
   // the update as a launch of its own, its 256-row stages dealt out to all
-  // SMs: where that leaves an SM fewer stages than the step kernel does (its
-  // CTAs update their own pairs, and SMs without a pair idle), by a margin for
+  // SMs: where that leaves an SM fewer stages than one wave of the step kernel does
+  // (its CTAs update their own pairs, and SMs without a pair idle), by a margin for
   // the second launch and the transforms' way through memory.  ms per call with
   // / without: 3072^2 (16 stages against 24) 323 / 372, 4864^2 without V (20
   // against 38) 1187 / 1511, 16384x256 (4 against 9) 23.1 / 24.7; but 4096x2048
-  // (11 against 12) 146 / 141, HSVD 2048x1024 (3 against 3) 30.4 / 28.1
+  // (11 against 12) 146 / 141, HSVD 2048x1024 (3 against 3) 30.4 / 28.1.  Over 37
+  // shapes of 16 to 288 pairs, with and without V, a sweep takes 0.68 to 1.00 of
+  // its time without (the most at 152 pairs, nothing where a stage or less is
+  // saved).  Waves are not counted: above two pairs per SM (9504 columns on 148
+  // SMs) the step kernel runs a second wave, dealt is never below the one wave's
+  // stages, and its CTAs go on updating their own pairs.
   if (vt && !one_launch && !p.variant && !g_pairs_per_cta) {
     const unsigned nst = (nrow + 255u) / 256u + (full ? (ncol + 255u) / 256u : 0u);
     const unsigned own = (p.width == 2u) ? 2u * nst : (nst + p.split - 1u) / p.split;

@@ -564,8 +564,12 @@ cudaError_t launch_l1_sweep(const bool sort, const bool accv, const StepParams &
 // rows: below, their thinner Gram shares and fewer update stages do not pay for
 // the wider exchange.  us per call of n = 256, ALG 11, with 8 / 4 CTAs per pair:
 // 256 rows 5256 / 5247, 512: 5470 / 5483, 1024: 5935 / 6444, 4096: 9394 / 10813,
-// 16384: 22471 / 28281.  More clusters than fit at once run in two waves: 34
-// pairs per step (2048 x 1088) take 104 ms with 4 CTAs per pair, 67 ms with 2.
+// 16384: 22471 / 28281.  us per sweep of other column counts (ALG 9): 1024 rows
+// x 32: 86 / 87, x 64: 150 / 153, x 128: 292 / 296, x 192: 435 / 442, x 320: 717 / 735, x
+// 448: 1001 / 1026; 8192 rows: 221 / 233, 383 / 422, 709 / 809, 1084 / 1231, 1831 /
+// 2090, 2537 / 3007; 512 rows: within 3 % either way.  More clusters than fit at
+// once run in two waves: 34 pairs per step (2048 x 1088) take 104 ms with 4 CTAs
+// per pair, 67 ms with 2; 16 pairs (1024 x 512) 2.05 ms a sweep with 8, 1.17 with 4.
 constexpr unsigned kSplit8Rows = 1024u;
 
 // how many clusters of N CTAs of the step kernel the current device holds at

@@ -143,9 +143,9 @@ inline size_t step_smem_bytes(const unsigned nsplit)
 // in the clusters a lane holds few chains of many operands shared, and lanes
 // 2j, 2j+1 share their columns y, all even (odd) lanes their columns x: 8
 // columns y per half-warp, in 8 bank groups.  Cycles per tile of the 3 warps of
-// a CTA: 1x1 643 (8 CTAs), 1x2 735 (4 CTAs), 2x2 1028 (2 CTAs); before, with 32
+// a CTA: 1x1 649 (8 CTAs), 1x2 768 (4 CTAs), 2x2 1093 (2 CTAs); before, with 32
 // columns y per warp, 2x1 864 (4 CTAs) and 4x1 1306 (2 CTAs).  With one CTA per
-// pair the chains fill 3 warps best as 4x2 with LX = 1 (1897; 2x2 on 4 warps
+// pair the chains fill 3 warps best as 4x2 with LX = 1 (1779; 2x2 on 4 warps
 // with the diagonal blocks beside other chains measured 25 % slower).
 // ---------------------------------------------------------------------------
 template <unsigned XU, unsigned YU, unsigned LX>

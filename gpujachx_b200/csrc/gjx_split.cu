@@ -1565,7 +1565,7 @@ int split_sweeps(const unsigned routine, const unsigned nrow, const unsigned nco
   // beside the next step's pair kernel, one CTA per block pair, on the SMs that
   // kernel leaves free: where those SMs do it in no more time than the pair
   // kernel takes (tiles of 8 K cycles against 2.5 K cycles per 64 rows of the
-  // Gram products and 130 K of the rest), else it would delay the next update.
+  // Gram products and 130 K of the rest, measured as 162 K), else it would delay the next update.
   // ms per call, beside / in one launch with G's: 4096^2 346 / 422 (64 CTAs of the
   // pair kernel), HSVD 1600x1344 59.4 / 62.0; 16384x5120 (80) 122 / 137 a sweep, but
   // 5120^2 is over the line.  A sweep of one step (64 columns) has no next pair
@@ -1678,9 +1678,10 @@ extern "C" int gjx_hypJacL2_split(const unsigned routine, const unsigned nrow, c
  * sp_pair_kernel launch of the last gjx_hypJacL2_split call to the end of:
  * [0] the Gram products, [1] the Gram epilogue, [2] the Cholesky factor,
  * [3] the inner sweeps, [4] the B operands; then CTA 0 of the update kernel
- * summed over the call: [5] waiting for its tile and B copies, [6] cutting
- * the tiles, [7] the products, [8] the epilogues, [9] items.  0 or
- * GJX_ERR_CUDA. */
+ * summed over the call: [5] the cutters waiting for the tensor core or the
+ * epilogue and issuing, [6] cutting the tiles, [7] the cutters waiting for
+ * copies, [8] the epilogues, [9] items (with V updated beside the next pair
+ * kernel CTA 0 of both launches).  0 or GJX_ERR_CUDA. */
 extern "C" int gjx_split_phase_cycles(long long *out10)
 {
   std::lock_guard<std::mutex> lk(gjx::g_split_mtx);

@@ -275,7 +275,10 @@ int gjx_hypJacL2_split(const unsigned routine, const unsigned nrow, const unsign
  * each warp group): [5] the cutters waiting for the tensor core or the
  * epilogue (digit planes or TMEM to be freed) and issuing the products, [6]
  * cutting tiles into digits, [7] the cutters waiting for copies (tiles, B
- * operands), [8] the epilogues, [9] the tiles it took.  0 or GJX_ERR_CUDA. */
+ * operands), [8] the epilogues, [9] the tiles it took; where V is updated by a
+ * launch of its own beside the next pair kernel, CTA 0 of both launches, which
+ * run at the same time, so that [5] to [8] are cycles of either per tile of [9].
+ * 0 or GJX_ERR_CUDA. */
 int gjx_split_phase_cycles(long long *out10);
 
 /* Frees the device buffers that hypJacL2 keeps between calls on the current
@@ -289,7 +292,11 @@ void gjx_set_verbose(const int level);
  * kernel launch with CUDA events on its stream; gjx_profile(0) resets and
  * stops timing (launch counts are always kept).  gjx_profile_read returns the
  * kernel launches since the reset (all kernels of this library), the
- * block-pair launches among them, and their summed device time in ms. */
+ * block-pair launches among them, and their summed device time in ms.  The
+ * time of a step whose update is a launch of its own is that of both launches.
+ * The split form's is that of its update kernel; while it is timed that kernel
+ * updates G and V, also where an untimed call updates V beside the next step's
+ * pair kernel (4096^2: 41.0 ms a sweep timed, 32.3 untimed). */
 void gjx_profile(const int enable);
 void gjx_profile_read(unsigned long long *launches, unsigned long long *l1_launches, double *l1_ms);
 
