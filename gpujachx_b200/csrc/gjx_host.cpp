@@ -58,11 +58,11 @@ std::mutex g_mtx;
 Strat g_strat;
 int g_verbose = 1;
 int g_sweep_mode = -1; // -1 automatic (the tuned choice, else per step), 0 per outer step, 1 one launch per sweep
-unsigned g_split = 0u;  // CTAs per block pair: 0 automatic (the tuned choice, else by the SM count), else 1, 2, 4
+unsigned g_split = 0u;  // CTAs per block pair: 0 automatic (the tuned choice, else l1_split), else 1, 2, 4, 8
 unsigned g_pairs_per_cta = 0u; // block pairs a CTA takes at a time: 0 automatic, 1, 2, or (batched form, two
                                // CTAs of 4 warps per SM) 3: one per CTA, 4: two per CTA
 unsigned g_variant = 0u; // pivot-block factor: 0 Gram + Cholesky, 1 QR (-DUSE_QR), 2 QR + Drmac (-DUSE_DRMAC)
-int g_batch_mode = -1;   // batched form: -1 the tuned choice (else per step), 0 one launch per step, 1 per sweep
+int g_batch_mode = -1;   // batched form: -1 the tuned choice (else run_batch's rule), 0 one launch per step, 1 per sweep
 unsigned g_batch_cap = 0u; // nonzero: the batched form stops after this many sweeps (the autotuner's runs)
 // the batched autotuner's choices, by the batch's sorted (nrow, ncol, signature) list
 std::map<std::vector<unsigned>, std::pair<unsigned, int>> g_batch_tuned; // (pairs per CTA, mode)

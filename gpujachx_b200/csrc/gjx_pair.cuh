@@ -113,7 +113,7 @@ __device__ __forceinline__ void inval_bars(uint64_t *const bars)
 
 inline size_t l1_smem_bytes() { return (size_t)kSmemDoubles * sizeof(double); }
 
-// the step kernels of 2- and 4-CTA clusters keep a third update buffer after
+// the step kernels of clusters keep a third update buffer after
 // the rest (128-byte aligned), 227 KB in all
 constexpr unsigned kOffUpd3 = (kSmemDoubles + 15u) & ~15u;
 constexpr unsigned kSmemDoubles3 = kOffUpd3 + kUpdStage;

@@ -99,8 +99,9 @@ int gjx_hypJacL2_batched(unsigned routine, unsigned nmat, const unsigned *nrow, 
  * launch per sweep, in which the block pairs of
  * consecutive outer steps start as soon as their two blocks are written
  * (used when all clusters of a step fit on the GPU at once, else per step;
- * measured no faster on a B200, kept for the autotuner).  The results are
- * the same bits either way. */
+ * with clusters of 4 where 8 CTAs would be the automatic choice; 1 % faster
+ * where the clusters fill the GPU, slower elsewhere, which the autotuner
+ * tells).  The results are the same bits either way. */
 void gjx_set_sweep_mode(int mode);
 
 /* CTAs per block pair (a thread-block cluster): 1, 2, 4 or 8 (8: launches per
